@@ -1,15 +1,14 @@
 // cimx_fused.cu — decides whether a pass list runs on the fast kernels
-// (cimx_fast.cuh, cimx_vol.cuh) and schedules them: a 3-D filter with short
+// (cimx_strip.cuh, cimx_vol.cuh) and schedules them: a 3-D filter with short
 // taps on all three axes is one launch of the volume kernel (k_vol);
-// otherwise passes along leading axes are streamed one launch each
-// (k_stream; the generic kernel for taps it does not cover), the passes
-// along the last two axes run fused in one slab launch (k_slab or
-// k_rowstream). Intermediates follow cuCIM's _run_1d_filters
-// ping-pong: every pass writes the output dtype, the last launch writes the
-// caller's output, one scratch buffer takes the others.
+// otherwise passes along leading axes are one launch each (k_columns; the
+// generic kernel for what it does not cover), the passes along the last two
+// axes run fused in one strip launch (k_strip) or, where their taps are long
+// or unequal, as a column launch and a strip launch. Intermediates follow
+// cuCIM's _run_1d_filters ping-pong: every pass writes the output dtype, the
+// last launch writes the caller's output, one scratch buffer takes the others.
 #include <algorithm>
 #include <cstring>
-#include <vector>
 
 #include "cimx_common.cuh"
 #include "cimx_fused.h"
@@ -25,16 +24,6 @@ bool fast_pair(int t, int d) {
     case DT_U8: return d == DT_F32 || d == DT_U8 || d == DT_U16;
     default: return false;
   }
-}
-
-// tap counts of the stream kernel's instantiations: the gaussians of
-// sigma 0.5 / 0.75 / 1 / 1.25 / 1.5 / 1.75 / 2 (truncate 4) and the short
-// box and derivative filters. Longer passes run faster on the generic
-// column kernel (measured along axis 0 of 256 x 512^2 float32: 19 / 25 taps
-// 303 / 583 us on the stream kernel, 250 / 263 us on k_cols_pairs).
-constexpr int kStreamMaxK = 17;
-bool stream_supports(int K) {
-  return K == 3 || K == 5 || K == 7 || K == 9 || K == 11 || K == 13 || K == 15 || K == 17;
 }
 
 struct Trimmed {
@@ -66,28 +55,52 @@ bool trim(const PassDesc& d, int max_k, Trimmed& t) {
 
 bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
-int launch_stream(const PassDesc& d, const Trimmed& t, int tin, const void* in, int tout,
-                  void* out, cudaStream_t st) {
+int launch_strip(const SlabArgs& a, int tin, int tout, cudaStream_t st) {
+  if (a.B == 0) return CIMX_OK;
   switch (tin) {
-    case DT_F32: return launch_stream_f32(d, t.w, t.K, t.anchor, t.interior_zero, in, tout, out, st);
-    case DT_U16: return launch_stream_u16(d, t.w, t.K, t.anchor, t.interior_zero, in, tout, out, st);
-    case DT_U8: return launch_stream_u8(d, t.w, t.K, t.anchor, t.interior_zero, in, tout, out, st);
+    case DT_F32: return launch_strip_f32(a, tout, st);
+    case DT_U16: return launch_strip_u16(a, tout, st);
+    case DT_U8: return launch_strip_u8(a, tout, st);
     default: return CIMX_FUSED_DECLINED;
   }
 }
 
-int launch_slab(SlabArgs& a, int tin, int tout, cudaStream_t st) {
+int launch_columns(const PassDesc& d, const Trimmed& t, int tin, const void* in, int tout,
+                   void* out, cudaStream_t st) {
+  if (d.outer * d.L * d.inner == 0) return CIMX_OK;
+  const bool skip = d.skip_zero && t.interior_zero;
   switch (tin) {
-    case DT_F32: return launch_slab_f32(a, tout, st);
-    case DT_U16: return launch_slab_u16(a, tout, st);
-    case DT_U8: return launch_slab_u8(a, tout, st);
+    case DT_F32: return launch_columns_f32(d, t.w, t.K, t.anchor, skip, in, tout, out, st);
+    case DT_U16: return launch_columns_u16(d, t.w, t.K, t.anchor, skip, in, tout, out, st);
+    case DT_U8: return launch_columns_u8(d, t.w, t.K, t.anchor, skip, in, tout, out, st);
     default: return CIMX_FUSED_DECLINED;
   }
+}
+
+// Extents the column and strip kernels take: narrower inner extents than 32
+// leave most of a warp's sectors unused, the strip works on 8 rows at a time,
+// and both index with 32 bits along an axis.
+constexpr int kColumnsMinInner = 32;
+constexpr int kStripMinRows = 4;
+constexpr int64_t kMaxExtent = 1LL << 30;
+
+// Whether the y and x passes share one strip launch. Fused, a value is read
+// and written once; apart, each pass has all registers and the y pass no x
+// halo. Measured on 256^3 float32, (y, x) fused against apart: 9 / 9 taps 42
+// against 58 us, 17 / 17 51 against 62, 33 / 33 71 against 83, 57 / 57 130
+// against 120; unequal counts (tested tap by tap when fused): 9 / 17 52
+// against 65, 33 / 17 96 against 78.
+bool strip_fuses(size_t elem, const PassDesc& dy, const Trimmed& y, const PassDesc& dx,
+                 const Trimmed& x) {
+  const int K = std::max(y.K, x.K);
+  if (K <= 17) return true;
+  if (K > 33 || kt_bound(elem, y.K) != kt_bound(elem, x.K)) return false;
+  return skip_kind(y.w, y.K, dy.skip_zero && y.interior_zero) < 2 &&
+         skip_kind(x.w, x.K, dx.skip_zero && x.interior_zero) < 2;
 }
 
 void fill_slab_pass(SlabPass& s, const PassDesc& d, const Trimmed& t, int pass_in) {
   s.K = t.K;
-  s.K8 = (t.K + 7) / 8 * 8;
   s.anchor = t.anchor;
   s.mode = d.mode;
   s.cval = d.cval;
@@ -150,7 +163,7 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
               int lib_flags, cudaStream_t st) {
   const int nd = in->ndim;
   const int D = out->dtype;
-  if (npasses < 1 || nd < 1) return CIMX_FUSED_DECLINED;
+  if (npasses < 1 || npasses > CIMX_MAX_NDIM || nd < 1) return CIMX_FUSED_DECLINED;
   // passes in strictly ascending axis order, float32 weights
   int prev_axis = -1;
   for (int i = 0; i < npasses; ++i) {
@@ -165,105 +178,105 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
     if (rc != CIMX_FUSED_DECLINED) return rc;
   }
 
-  // leading axes are streamed, the last two axes go to the slab kernel
-  const int ylast = nd >= 2 ? nd - 2 : -1;
-  std::vector<int> lead, tail;
-  for (int i = 0; i < npasses; ++i) (ds[i].axis < ylast ? lead : tail).push_back(i);
-
-  std::vector<Trimmed> tr(npasses);
-  // a leading pass the stream kernel does not cover (longer taps, rows not
-  // a multiple of 4) runs on the generic kernel: worthwhile while the last
-  // two axes still take one slab launch
-  std::vector<char> lead_generic(npasses, 0);
-  for (size_t n = 0; n < lead.size(); ++n) {
-    const int i = lead[n];
-    const int tin = n == 0 ? in->dtype : D;
-    const bool stream_ok = !(lib_flags & CIMX_L_NO_STREAM) && trim(ds[i], kStreamMaxK, tr[i]) &&
-                           stream_supports(tr[i].K) && fast_pair(tin, D) &&
-                           ds[i].inner % 4 == 0;
-    if (!stream_ok) {
-      if (tail.empty()) return CIMX_FUSED_DECLINED;
-      lead_generic[i] = 1;
+  // The launches, in order: one per leading axis (in columns, or generic),
+  // then one or two for the last two axes.
+  enum Kind { kColumns, kGeneric, kStrip };
+  struct Step {
+    Kind kind;
+    int y, x;  // the passes it takes; kStrip: y is -1 for a lone x pass
+  };
+  Step steps[CIMX_MAX_NDIM];
+  Trimmed tr[CIMX_MAX_NDIM];
+  int nl = 0;  // launches
+  int64_t n = 1, longest = 0;
+  for (int k = 0; k < nd; ++k) {
+    n *= in->shape[k];
+    longest = std::max<int64_t>(longest, in->shape[k]);
+  }
+  if (longest >= kMaxExtent) return CIMX_FUSED_DECLINED;
+  auto plan = [&](bool fuse_all) {
+    bool fast = false;  // any launch that the generic kernels would not make
+    nl = 0;
+    for (int i = 0; i < npasses; ++i) {
+      const int tin = i == 0 ? in->dtype : D;
+      Step s{kGeneric, i, -1};
+      if (nd >= 2 && fast_pair(tin, D) && trim(ds[i], kSlabMaxK, tr[i])) {
+        if (ds[i].axis == nd - 1) {
+          if (n / std::max<int64_t>(1, in->shape[nd - 1]) >= kStripMinRows) s = {kStrip, -1, i};
+        } else if (ds[i].axis == nd - 2 && i + 1 < npasses &&
+                   trim(ds[i + 1], kSlabMaxK, tr[i + 1]) &&
+                   (fuse_all || strip_fuses(dtype_size(tin), ds[i], tr[i], ds[i + 1], tr[i + 1]))) {
+          s = {kStrip, i, i + 1};
+          ++i;
+        } else if (ds[i].inner >= kColumnsMinInner &&
+                   (ds[i].axis == nd - 2 || !(lib_flags & CIMX_L_NO_STREAM))) {
+          s.kind = kColumns;
+        }
+      }
+      fast |= s.kind != kGeneric;
+      steps[nl++] = s;
     }
-  }
-  const int tail_in = lead.empty() ? in->dtype : D;
-  // a lone pass along the last axis over float32 data runs on the slab
-  // kernel behind an identity y pass (one tap of 1: fma(v, 1, +0) = v, kept
-  // as float32, exact). A -0 input becomes +0, which the x pass's chain from
-  // +0 cannot tell apart. Measured on 16 x 2048 x 2048 with 9 taps: 148 us
-  // against 266 us on the generic row kernel. For 8- and 16-bit input the
-  // generic row kernel is the faster (uint16: 240 us against 316 us).
-  const bool y_identity = !tail.empty() && nd >= 2 && ds[tail[0]].axis == nd - 1 &&
-                          tail_in == DT_F32 && D == DT_F32;
-  if (!tail.empty()) {
-    // the slab kernel needs a pass along the second-to-last axis
-    if (nd < 2 || (ds[tail[0]].axis != nd - 2 && !y_identity)) return CIMX_FUSED_DECLINED;
-    if (!fast_pair(tail_in, D)) return CIMX_FUSED_DECLINED;
-    for (int i : tail)
-      if (!trim(ds[i], kSlabMaxK, tr[i])) return CIMX_FUSED_DECLINED;
-  }
-  const size_t vec_in = 4 * dtype_size(in->dtype), vec_out = 4 * dtype_size(D);
-  if (!aligned(in->data, vec_in) || !aligned(out->data, vec_out)) return CIMX_FUSED_DECLINED;
+    return fast;
+  };
+  if (!plan(false)) return CIMX_FUSED_DECLINED;
 
   // ping-pong schedule: the last launch writes `out`
-  const int nl = (int)lead.size() + (tail.empty() ? 0 : 1);
-  int64_t n = 1;
-  for (int k = 0; k < nd; ++k) n *= in->shape[k];
   const size_t tbytes = (size_t)n * dtype_size(D);
   void* temp = nullptr;
   if (nl >= 2) {
     temp = scratch_alloc(tbytes, st);
-    if (!temp) return fail(CIMX_E_NOMEM, "scratch allocation for the ping-pong buffer failed");
+    // without scratch memory, both tail passes in one launch whatever their taps
+    if (!temp && (!plan(true) || nl >= 2))
+      return fail(CIMX_E_NOMEM, "scratch allocation for the ping-pong buffer failed");
   }
-  auto dst_of = [&](int j) { return ((nl - 1 - j) % 2 == 0) ? out->data : temp; };
-
   int rc = CIMX_OK;
   const void* src = in->data;
   int tsrc = in->dtype;
-  int j = 0;
-  for (int i : lead) {
-    void* dst = dst_of(j++);
-    if (lead_generic[i]) {
-      PassDesc d = ds[i];
-      d.in = src;
-      d.out = dst;
-      d.tin = tsrc;
-      d.tout = D;
-      rc = launch_generic_pass(d, st);
-    } else {
-      rc = launch_stream(ds[i], tr[i], tsrc, src, D, dst, st);
+  for (int j = 0; j < nl && rc == CIMX_OK; ++j) {
+    const Step& s = steps[j];
+    void* dst = ((nl - 1 - j) % 2 == 0) ? out->data : temp;
+    switch (s.kind) {
+      case kColumns: rc = launch_columns(ds[s.y], tr[s.y], tsrc, src, D, dst, st); break;
+      case kGeneric: {
+        PassDesc d = ds[s.y];
+        d.in = src;
+        d.out = dst;
+        d.tin = tsrc;
+        d.tout = D;
+        rc = launch_generic_pass(d, st);
+        break;
+      }
+      default: {
+        SlabArgs a{};
+        a.in = src;
+        a.out = dst;
+        a.X = in->shape[nd - 1];
+        a.Y = in->shape[nd - 2];
+        a.B = (a.X * a.Y == 0) ? 0 : n / (a.X * a.Y);
+        int pass_in = tsrc;
+        if (s.y >= 0) {
+          fill_slab_pass(a.py, ds[s.y], tr[s.y], pass_in);
+          a.has_y = 1;
+          pass_in = D;
+        } else {
+          // the x pass alone: all rows of the array as one slab, staged by an
+          // identity y pass
+          if (a.B * a.Y < kMaxExtent) {
+            a.Y *= a.B;
+            a.B = 1;
+          }
+          a.py.K = 1;
+          a.py.mode = CIMX_MODE_NEAREST;  // no halo: K = 1, anchor 0
+          a.py.dt = pass_in;
+          a.py.w[0] = 1.f;
+        }
+        a.has_x = 1;
+        fill_slab_pass(a.px, ds[s.x], tr[s.x], pass_in);
+        rc = launch_strip(a, tsrc, D, st);
+      }
     }
-    if (rc != CIMX_OK) break;
     src = dst;
     tsrc = D;
-  }
-  if (rc == CIMX_OK && !tail.empty()) {
-    SlabArgs a{};
-    a.no_rowstream = (lib_flags & CIMX_L_NO_ROWSTREAM) ? 1 : 0;
-    static const int kSpans[4] = {0, 1, 2, 8};
-    a.span = kSpans[(lib_flags >> CIMX_L_SLAB_SPAN_SHIFT) & 3];
-    a.in = src;
-    a.out = dst_of(j++);
-    a.X = in->shape[nd - 1];
-    a.Y = nd >= 2 ? in->shape[nd - 2] : 1;
-    a.B = (a.X * a.Y == 0) ? 0 : n / (a.X * a.Y);
-    int pass_in = tsrc;
-    if (y_identity) {
-      a.py = SlabPass{};
-      a.py.K = 1;
-      a.py.K8 = 8;
-      a.py.mode = CIMX_MODE_NEAREST;  // no halo: K = 1, anchor 0
-      a.py.dt = pass_in;
-      a.py.w[0] = 1.f;
-      a.has_y = 1;
-    }
-    for (int i : tail) {
-      const bool is_x = ds[i].axis == nd - 1;
-      fill_slab_pass(is_x ? a.px : a.py, ds[i], tr[i], pass_in);
-      (is_x ? a.has_x : a.has_y) = 1;
-      pass_in = D;
-    }
-    rc = launch_slab(a, tsrc, D, st);
   }
   scratch_free(temp, tbytes, st);
   // every check that can decline ran before the first launch

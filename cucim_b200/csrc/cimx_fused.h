@@ -1,5 +1,6 @@
-// cimx_fused.h — entry into the fast kernels of the plain path
-// (cimx_fast.cuh, instantiated per input dtype in cimx_fast_{f32,u16,u8}.cu)
+// cimx_fused.h — entry into the fast kernels of the plain path (cimx_vol.cuh
+// and cimx_strip.cuh, instantiated per input dtype in
+// cimx_{fast,strip}_{f32,u16,u8}.cu)
 // and the dispatcher that decides whether a pass list can use them
 // (cimx_fused.cu).
 #pragma once
@@ -12,11 +13,11 @@ namespace cimx {
 // then runs the passes one launch at a time.
 constexpr int CIMX_FUSED_DECLINED = 1;
 
-constexpr int kSlabMaxK = 64;  // longest pass the slab kernel takes
+constexpr int kSlabMaxK = 65;  // longest pass the strip and column kernels take
 
-// One pass of the slab kernel (float32 weights, already trimmed).
+// One pass of the strip and volume kernels (float32 weights, already trimmed).
 struct SlabPass {
-  int K, K8, anchor, mode;
+  int K, anchor, mode;
   double cval;
   int cval_as_input, dt, skip, pad;
   float w[kSlabMaxK];
@@ -26,11 +27,7 @@ struct SlabArgs {
   const void* in;
   void* out;
   long long B, Y, X;
-  long long tiles_x, tiles_y;
-  int has_y, has_x;
-  int* status;  // device status word for bounded waits
-  int no_rowstream;  // CIMX_L_NO_ROWSTREAM: always the slab kernel
-  int span;          // slabs per CTA (float input with TMA); 0: about four
+  int has_y, has_x;  // has_y 0: py is the identity (one tap of 1)
   SlabPass py, px;
 };
 
@@ -44,6 +41,23 @@ struct VolArgs {
   SlabPass pz, py, px;
 };
 
+// Tap-count bounds of the strip kernels' instantiations (cimx_strip.cuh): steps
+// of four for float32 (every gaussian length is odd, the most common are
+// bounds themselves), of eight for the integer types.
+constexpr int kt_step(size_t elem) { return elem == 4 ? 4 : 8; }
+constexpr int kt_bound(size_t elem, int K) {
+  return K <= 5 ? 5 : K <= 9 ? 9 : 9 + (K - 9 + kt_step(elem) - 1) / kt_step(elem) * kt_step(elem);
+}
+
+// What the skip rule leaves out of a pass: 0 nothing, 1 only the centre tap
+// (an odd Gaussian derivative), 2 others.
+inline int skip_kind(const float* w, int K, bool skip) {
+  if (!skip) return 0;
+  for (int k = 0; k < K; ++k)
+    if (w[k] == 0.f && k != K / 2) return 2;
+  return (K & 1) ? 1 : 2;
+}
+
 // Runs the whole pass list `ds` (already resolved against the input shape)
 // in fast launches when they cover it. Returns CIMX_OK, a negative error, or
 // CIMX_FUSED_DECLINED (nothing was launched).
@@ -54,22 +68,21 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
 int launch_copy_cast(const void* in, int tin, void* out, int tout, int64_t n,
                      cudaStream_t stream);
 
-// stream pass along a strided axis, by input dtype; K in {3,5,...,17} (odd)
-int launch_stream_f32(const PassDesc& d, const float* w, int K, int anchor, bool interior_zero,
-                      const void* in, int tout, void* out, cudaStream_t st);
-int launch_stream_u16(const PassDesc& d, const float* w, int K, int anchor, bool interior_zero,
-                      const void* in, int tout, void* out, cudaStream_t st);
-int launch_stream_u8(const PassDesc& d, const float* w, int K, int anchor, bool interior_zero,
-                     const void* in, int tout, void* out, cudaStream_t st);
-
 // single-launch 3-D filter, by input dtype; equal K in {3, 5} on every axis
 int launch_vol_f32(const VolArgs& v, int tout, cudaStream_t st);
 int launch_vol_u16(const VolArgs& v, int tout, cudaStream_t st);
 int launch_vol_u8(const VolArgs& v, int tout, cudaStream_t st);
 
-// fused (y, x) slab launch, by input dtype
-int launch_slab_f32(SlabArgs& a, int tout, cudaStream_t st);
-int launch_slab_u16(SlabArgs& a, int tout, cudaStream_t st);
-int launch_slab_u8(SlabArgs& a, int tout, cudaStream_t st);
+// the last two axes (or the last alone) in one launch, and one pass along a
+// strided axis, by input dtype; up to kSlabMaxK taps
+int launch_strip_f32(const SlabArgs& a, int tout, cudaStream_t st);
+int launch_columns_f32(const PassDesc& d, const float* w, int K, int anchor, bool skip,
+                       const void* in, int tout, void* out, cudaStream_t st);
+int launch_strip_u16(const SlabArgs& a, int tout, cudaStream_t st);
+int launch_columns_u16(const PassDesc& d, const float* w, int K, int anchor, bool skip,
+                       const void* in, int tout, void* out, cudaStream_t st);
+int launch_strip_u8(const SlabArgs& a, int tout, cudaStream_t st);
+int launch_columns_u8(const PassDesc& d, const float* w, int K, int anchor, bool skip,
+                      const void* in, int tout, void* out, cudaStream_t st);
 
 }  // namespace cimx

@@ -1,11 +1,10 @@
 // cimx_tune.cu — the schedule autotuner of cimx_separable.
 //
 // A pass list can run on several kernel schedules that give bit-identical
-// results: the single-launch volume kernel or stream + slab launches, the
-// stream kernel or the generic kernel for leading axes, the row stream or
-// the slab kernel for the last two axes, the volume kernel's z chunk, fused
-// launches or one launch per pass. Which is fastest depends on the dtypes,
-// the tap counts and the extents. (cuCIM makes the corresponding choice, its
+// results: the single-launch volume kernel or column + strip launches, the
+// column kernel or the generic kernel for leading axes, the volume kernel's z
+// chunk, fused launches or one launch per pass. Which is fastest depends on
+// the dtypes, the tap counts and the extents. (cuCIM makes the corresponding choice, its
 // shared-memory or elementwise kernel, by a fixed rule:
 // _vendored/_ndimage_filters.py:284-297.) With algorithm="tensor" the
 // tuner also chooses between the tensor-core and the plain float32 pass per
@@ -439,17 +438,12 @@ int tuned_flags(const std::string& key, int lib_flags, cudaStream_t st,
   const int base = lib_flags & ~(kScheduleBits | CIMX_L_NO_TUNE);
   const int sched[] = {0,
                        CIMX_L_NO_VOLUME,
-                       CIMX_L_NO_ROWSTREAM,
-                       CIMX_L_NO_VOLUME | CIMX_L_NO_ROWSTREAM,
                        CIMX_L_NO_STREAM,
                        CIMX_L_NO_STREAM | CIMX_L_NO_VOLUME,
                        CIMX_L_NO_FUSION,
                        1 << CIMX_L_ZCHUNK_SHIFT,
                        2 << CIMX_L_ZCHUNK_SHIFT,
-                       3 << CIMX_L_ZCHUNK_SHIFT,
-                       1 << CIMX_L_SLAB_SPAN_SHIFT,
-                       2 << CIMX_L_SLAB_SPAN_SHIFT,
-                       3 << CIMX_L_SLAB_SPAN_SHIFT};
+                       3 << CIMX_L_ZCHUNK_SHIFT};
   for (int s : sched) cands.push_back(base | s);
   if (base & kTensorBits) {
     cands.push_back(base | CIMX_L_TENSOR_ALL_LINES);

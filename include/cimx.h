@@ -92,15 +92,14 @@ enum {
                                    cores whatever its line length (testing, measurement) */
   /* Schedule choices. Each selects between kernels that give bit-identical
    * results; the autotuner (cimx_tune_*) picks among them per call signature. */
-  CIMX_L_NO_VOLUME = 1 << 4,    /* 3-D short filters: stream + slab launches instead of the
-                                   single-launch volume kernel */
-  CIMX_L_NO_STREAM = 1 << 5,    /* leading-axis passes on the generic kernel, not k_stream */
-  CIMX_L_NO_ROWSTREAM = 1 << 6, /* (y, x) passes on the slab kernel, not the row stream */
+  CIMX_L_NO_VOLUME = 1 << 4,    /* 3-D short filters: column + strip launches instead of
+                                   the single-launch volume kernel */
+  CIMX_L_NO_STREAM = 1 << 5,    /* leading-axis passes on the generic kernel, not k_columns */
+  CIMX_L_NO_ROWSTREAM = 1 << 6, /* no effect (accepted for recorded schedules) */
   CIMX_L_NO_TUNE = 1 << 7,      /* this call neither consults nor fills the tuning table */
   CIMX_L_ZCHUNK_SHIFT = 8,      /* bits 8-9: volume-kernel z chunk, 0 = automatic,
                                    1/2/3 = 32/64/128 slices */
-  CIMX_L_SLAB_SPAN_SHIFT = 10,  /* bits 10-11: slabs each slab-kernel CTA walks (float
-                                   input), 0 = automatic (about 4), 1/2/3 = 1/2/8 */
+  CIMX_L_SLAB_SPAN_SHIFT = 10,  /* bits 10-11: no effect (accepted for recorded schedules) */
 };
 
 /* One 1-D correlation pass of a separable filter. */
@@ -155,7 +154,7 @@ CIMX_API int cimx_set_allocator(cimx_alloc_fn alloc, cimx_free_fn release, void*
 
 /* The schedule autotuner of cimx_separable (and of every entry built on
  * it). A pass list can run on several kernel schedules with bit-identical
- * results (CIMX_L_NO_VOLUME, CIMX_L_NO_STREAM, CIMX_L_NO_ROWSTREAM,
+ * results (CIMX_L_NO_VOLUME, CIMX_L_NO_STREAM,
  * CIMX_L_NO_FUSION, the z chunk bits); with a tensor flag the tensor-core
  * and plain passes are candidates too. The tuner keys a table on the call
  * signature (dtypes, shape, each pass's axis, taps, anchor, mode and flags,

@@ -1,0 +1,140 @@
+"""The strip and column kernels (csrc/cimx_strip.cuh) against the oracle, bit
+for bit, where their geometry changes: around a group of 8 rows, a tile's
+columns, the tap-count bounds, unequal and partly zero taps, odd row lengths
+and base addresses, axes shorter than the taps."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import restate as R
+
+pytestmark = pytest.mark.gpu
+
+MODES = ["reflect", "mirror", "nearest", "constant", "wrap"]
+PAIRS = [("float32", "float32"), ("uint16", "float32"), ("uint16", "uint16"),
+         ("uint8", "float32"), ("uint8", "uint8"), ("uint8", "uint16")]
+
+
+@pytest.fixture(scope="module")
+def ndi(cuda):
+    from cucim_b200 import ndimage
+
+    return ndimage
+
+
+def _data(shape, dtype, seed=0):
+    r = np.random.default_rng(seed)
+    if dtype == "float32":
+        return r.standard_normal(shape).astype(np.float32)
+    return r.integers(0, np.iinfo(dtype).max + 1, shape).astype(dtype)
+
+
+def _taps(K, kind, seed=0):
+    """plain: positive, sum 1; signed: any sign, sum of magnitudes 2 (integer
+    outputs wrap or saturate); centre / holes: zeros the skip rule leaves out."""
+    w = np.random.default_rng(seed + K).random(K) + 0.1
+    if kind == "signed":
+        w *= np.where(np.arange(K) % 3, 1, -1) * 2
+    w /= np.abs(w).sum() / (2 if kind == "signed" else 1)
+    if kind == "centre":
+        w[K // 2] = 0
+    if kind == "holes":
+        w[1::3] = 0
+    return w
+
+
+def _run(ndi, x, passes, output, **kw):
+    """The passes as one call of the library, and one by one in the oracle."""
+    xd = torch.as_tensor(x).cuda()
+    got = ndi._run(xd, [(ax, w, m, o, False) for ax, w, m, o in passes], np.dtype(output),
+                   kw.get("cval", 0.0))
+    exp = x
+    for ax, w, m, o in passes:
+        exp = R.correlate1d(exp, w, ax, output=np.dtype(output), mode=m, origin=o,
+                            cval=kw.get("cval", 0.0))
+    np.testing.assert_array_equal(got.cpu().numpy(), exp)
+
+
+@pytest.mark.parametrize("pair", PAIRS, ids=lambda p: "-".join(p))
+@pytest.mark.parametrize("K", [2, 5, 6, 9, 10, 13, 17, 18, 25, 32, 33, 34, 41, 57, 65])
+def test_tap_bounds(ndi, pair, K):
+    """Both tail passes (fused or apart) and each alone, at every tap bound."""
+    x = _data((2, 37, 75), pair[0], K)
+    for kind in ("plain", "signed"):
+        w = _taps(K, kind)
+        for mode in ("reflect", "constant"):
+            _run(ndi, x, [(1, w, mode, 0), (2, w, mode, 0)], pair[1], cval=3.0)
+            _run(ndi, x, [(1, w, mode, 0)], pair[1], cval=3.0)
+            _run(ndi, x, [(2, w, mode, 0)], pair[1], cval=3.0)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("ky,kx", [(1, 9), (9, 3), (17, 5), (8, 17), (33, 9), (18, 33), (65, 21)])
+def test_unequal_and_zero_taps(ndi, mode, ky, kx):
+    """Unequal counts, a zero centre tap and zeros between taps, with values
+    that make a skipped tap matter, origins and a fill value."""
+    x = _data((3, 30, 53), "float32", ky)
+    x[0, 5, 7], x[1, 20, 50], x[2, 0, 0] = np.inf, np.nan, -np.inf
+    for kind in ("plain", "centre", "holes"):
+        wy, wx = _taps(ky, kind), _taps(kx, kind)
+        if not (wy.any() and wx.any()):
+            continue
+        _run(ndi, x, [(1, wy, mode, 0), (2, wx, mode, 0)], "float32", cval=1.5)
+        _run(ndi, x, [(1, wy, mode, (ky - 1) // 2), (2, wx, mode, -(kx // 2))], "float32",
+             cval=np.inf if mode == "constant" else 0.0)
+        _run(ndi, x, [(0, wx, mode, 0)], "float32", cval=-2.0)
+
+
+@pytest.mark.parametrize("rows", [1, 3, 7, 8, 9, 16, 23])
+@pytest.mark.parametrize("cols", [1, 2, 31, 32, 112, 113, 496, 497, 504, 1021])
+def test_tile_edges(ndi, rows, cols):
+    """Rows around the group of 8, columns around the tile widths; 17 taps
+    are longer than the short axes, whose halo folds more than once."""
+    w = _taps(17, "plain")
+    for mode in MODES:
+        x = _data((2, rows, cols), "float32", rows * cols)
+        _run(ndi, x, [(1, w, mode, 0), (2, w, mode, 0)], "float32", cval=2.0)
+    x = _data((2, rows, cols), "uint16", rows * cols)
+    _run(ndi, x, [(1, w, "mirror", 0), (2, w, "wrap", 0)], "uint16")
+    _run(ndi, x, [(0, w[:5], "reflect", 0), (2, w, "nearest", 0)], "uint16")
+
+
+@pytest.mark.parametrize("pair", PAIRS, ids=lambda p: "-".join(p))
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_base_alignment(ndi, pair, offset):
+    """Contiguous arrays whose first element lies off the vector boundary."""
+    shape, w = (4, 19, 64), _taps(9, "plain")
+    n = int(np.prod(shape))
+    flat = _data(n + 4, pair[0], offset)
+    x = flat[offset:offset + n].reshape(shape)
+    xd = torch.as_tensor(flat).cuda()[offset:offset + n].view(shape)
+    out = torch.empty(n + 4, dtype=ndi._arrays.torch_dtype(np.dtype(pair[1])),
+                      device="cuda")[4 - offset:n + 4 - offset].view(shape)
+    exp = x
+    for ax in (1, 2):
+        exp = R.correlate1d(exp, w, ax, output=np.dtype(pair[1]), mode="reflect")
+    ndi._run(xd, [(1, w, "reflect", 0, False), (2, w, "reflect", 0, False)], out, 0.0)
+    np.testing.assert_array_equal(out.cpu().numpy(), exp)
+
+
+def test_long_tail_passes_without_scratch_memory(ndi):
+    """Tail passes too long to share a launch take scratch memory; where there
+    is none they run as one launch all the same."""
+    import ctypes
+
+    from cucim_b200 import _lib
+
+    fn = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p)
+    rel = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p,
+                           ctypes.c_void_p)
+    refuse, ignore = fn(lambda *a: None), rel(lambda *a: None)
+    set_allocator = _lib.lib.cimx_set_allocator
+    set_allocator(ctypes.cast(refuse, ctypes.c_void_p), ctypes.cast(ignore, ctypes.c_void_p), None)
+    try:
+        for ky, kx in ((57, 57), (33, 9), (64, 33)):
+            _run(ndi, _data((3, 40, 70), "float32"),
+                 [(1, _taps(ky, "centre"), "reflect", 0), (2, _taps(kx, "holes"), "wrap", 0)],
+                 "float32")
+    finally:
+        set_allocator(None, None, None)
