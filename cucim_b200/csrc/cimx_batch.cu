@@ -14,26 +14,47 @@
 //           'reflect' borders, float32 intermediates;
 //   out   = sqrt(d0*d0 + d1*d1), each product and the sum rounded to float32.
 //
-// Work: the tiles' 64 x 64 output blocks form one flat list (each tile knows
-// the index of its first block); CTAs (three per SM up to a radius of about
-// 38) walk the list with a grid stride. A block computes its gray halo
-// region ((64 + 2 + 2r) rows) in strips of 28 columns through two
-// shared-memory buffers, the next strip's loads in flight during the current
-// strip's y pass into T; then the x pass into S (over the strip buffers),
-// and the edge, smoothing and magnitude steps per 4 outputs in registers.
+// Work: a tile is cut into strips of up to 254 - 2r output columns and chunks
+// of up to 254 rows; a CTA walks down a strip, 16 rows at a time, on 256
+// staged columns:
+//   * gray rows live in a ring in shared memory, the K - 1 + 16 rows that a
+//     group's y chains read: every pixel is converted once per strip (1.1 to
+//     1.35 times in all, for the halo columns) and its words are loaded while
+//     the previous group is filtered;
+//   * y chains: a thread takes a column pair and 8 rows, the rows streaming
+//     through a register window in blocks of 8 (ring slots in multiples of 8:
+//     a block never wraps), one f32x2 FMA per tap and pair;
+//   * x chains: a thread takes a row pair and 8 columns of the result;
+//   * edges and magnitude: a thread takes one column and 4 rows, so that a
+//     warp's stores cover consecutive floats at any alignment.
+// Two barriers per 16 rows, two CTAs per SM up to 65 taps (113 KB each, set by
+// the batch's largest radius).
+//
+// Bound: instruction issue, shared between the FMAs (about K (1 + 256 /
+// (254 - 2r)) per pixel) and the conversion and edge arithmetic (about 100
+// instructions per pixel), at 16 warps per SM with barriers (51 % of the issue
+// slots used). 1024 tiles of 64-1024 a side, sigmas 0.5-8: 3.15 ms; 64 x 64
+// blocks with a halo on all sides, whose gray region is 2.3 times the output
+// at 33 taps and 4.1 at 65, 6.99; chunks of 254 instead of 510 rows and
+// single-row edges 3.52.
 // The launch reads only device memory that the caller prepared, so it can
 // be captured in a CUDA graph and replayed.
 #include <algorithm>
 #include <mutex>
 
 #include "cimx_common.cuh"
+#include "cimx_fast.cuh"
 #include "cimx_internal.h"
 
 namespace cimx {
 namespace {
 
-constexpr int kBT = 64;          // output block side
+constexpr int kBT = 64;          // side of the blocks that the tile table counts
 constexpr int kBThreads = 256;
+constexpr int kBCols = 256;      // staged columns of a strip
+constexpr int kBG = 16;          // rows per group
+constexpr int kBRows = 32 * kBG - 2;  // output rows per chunk: 32 groups with the edge passes' halo
+constexpr int kBSRows = kBG + 2;      // smoothed rows kept for the edge passes
 constexpr int kBMaxTaps = 129;   // radius <= 64
 static_assert(sizeof(CimxBatchTile) == 56, "CimxBatchTile layout is part of the ABI");
 
@@ -48,349 +69,389 @@ struct BatchArgs {
 
 __device__ __forceinline__ int nearest_idx(int i, int n) { return i < 0 ? 0 : (i >= n ? n - 1 : i); }
 
-// The float64 value of one channel, (double)((float)u * (float)(1/255)),
-// computed without a table (a table's random reads conflicted on the
-// shared-memory banks): float(u) exactly, the float32 product, then the
-// float widened by rebiasing its exponent (the value is 0 or normal)
-__device__ __forceinline__ double chan(uint32_t u) {
-  const float f = __fmul_rn(__fsub_rn(__uint_as_float(0x4B000000u | u), 8388608.0f),
-                            static_cast<float>(1.0 / 255.0));
-  const unsigned long long b = __float_as_uint(f);
-  return __longlong_as_double(
-      b ? static_cast<long long>((b << 29) + (static_cast<unsigned long long>(1023 - 127) << 52))
-        : 0ll);
+// gray = (float)(0.0721 b + (0.2125 r + 0.7154 g)) in float64 fused
+// multiply-adds, in the order in which the per-tile rgb2gray kernel contracts
+// them, of three bytes. A channel is (double)((float)u * (float)(1 / 255)):
+// with c = (float)(1 / 255), 2^23 + u is a float and 2^23 c is one too, so one
+// FMA, (2^23 + u) c - 2^23 c, gives u c rounded once; the float is widened by
+// rebiasing its exponent (the conversion unit is a sixteenth of the FMA rate, a
+// table's random reads conflict on the banks). That makes 2^-127 of a zero,
+// which vanishes beside any other channel; black pixels are put right at the
+// end.
+__device__ __forceinline__ float luma(uint32_t r, uint32_t g, uint32_t b) {
+  auto chan = [](uint32_t u) {
+    constexpr float c = static_cast<float>(1.0 / 255.0);
+    const uint32_t f = __float_as_uint(fmaf(__uint_as_float(0x4B000000u | u), c, -8388608.0f * c));
+    return __hiloint2double(static_cast<int>((f >> 3) + ((1023u - 127u) << 20)),
+                            static_cast<int>(f << 29));
+  };
+  const float v = __double2float_rn(
+      __fma_rn(0.0721, chan(b), __fma_rn(0.2125, chan(r), __dmul_rn(0.7154, chan(g)))));
+  return (r | g | b) ? v : 0.f;
 }
 
-// gray = (float)(0.2125 r + 0.7154 g + 0.0721 b) with the float64
-// operations in the order the per-tile rgb2gray kernel contracts them:
-// 0.0721 b + (0.2125 r + 0.7154 g), each sum a fused multiply-add.
-__device__ __forceinline__ float luma_f64(double r, double g, double b) {
-  return __double2float_rn(__fma_rn(0.0721, b, __fma_rn(0.2125, r, __dmul_rn(0.7154, g))));
-}
+using fast::f2;
+using fast::fma2;
+using fast::hi2;
+using fast::lo2;
+using fast::pack2;
 
-constexpr int kSS = kBT + 3;  // row stride of S: odd, for the column-wise writes of the x pass
-constexpr int kGB = 4;  // 4-pixel groups whose words a thread loads at once (gray step)
-constexpr int kCW = 28;  // gray-region columns per strip: 9 x 28 y-pass items fill 256 threads once
-constexpr int kCG = kCW / 4;  // 4-pixel groups per strip row
-constexpr int kSlack = 16;    // spare strip rows: the chains may read 2 x 8 - 1 rows past the last
-constexpr int kBR = 8;  // outputs per thread in the Gaussian passes
-constexpr int kBG = (kBT + 2 + kBR - 1) / kBR;  // 8-output groups over 66 rows or columns
-
-// Shared-memory areas for the batch's largest radius (floats). A: two gray
-// strips of (64 + 2 + 2 max_r + kSlack) rows x kCW, or S (66 x kSS). B: T
-// (66 rows x the odd stride 64 + 3 + 2 max_r, 64 spare floats for the x
-// chains' reads past the last row).
-__host__ __device__ inline int batch_area_a(int max_r) {
-  const int strips = 2 * (kBT + 2 + 2 * max_r + kSlack) * kCW;
-  return strips > (kBT + 2) * kSS ? strips : (kBT + 2) * kSS;
+// Shared memory of one CTA, in this order: taps as (w, w) pairs; the gray ring,
+// a multiple of 8 rows that covers the K - 1 + kBG rows of one group's chains;
+// T, the group's y results as row pairs, 16 spare bytes per row pair so that 8
+// row pairs hit distinct banks; S, kBSRows smoothed rows as a ring of row pairs.
+// The x chains read up to 16 columns past a row pair: values that no stored
+// output uses, the last of them in S.
+constexpr int kTapBytes = (kBMaxTaps + 1) * 8;
+constexpr int kTPitch = kBCols * 8 + 16;
+constexpr int kTBytes = kBG / 2 * kTPitch;
+__host__ __device__ constexpr int ring_rows(int K) { return (K - 1 + 7) / 8 * 8 + kBG; }
+__host__ __device__ constexpr int s_pitch(int K) { return (kBCols - (K - 1) + 7) / 8 * 8 + 4; }
+// for K taps and fewer: S is widest for the shortest filter with K's ring, and
+// the next longer ring adds 8 KB against 8 columns of S
+__host__ __device__ constexpr int batch_smem(int K) {
+  const int widest = kBCols + 8 - (K - 1 + 7) / 8 * 8 + 4;
+  return kTapBytes + ring_rows(K) * kBCols * 4 + kTBytes + kBSRows * widest * 4;
 }
-__host__ __device__ inline int batch_area_b(int max_r) {
-  return (kBT + 2) * (kBT + 3 + 2 * max_r) + 64;
-}
+static_assert(batch_smem(65) <= 113 * 1024 - 256, "two CTAs per SM up to 65 taps");
+static_assert(batch_smem(kBMaxTaps) <= 223 * 1024, "longest filter");
+static_assert(kBCols - (kBMaxTaps - 1) - 2 >= kBT && kBRows >= kBT,
+              "a tile has no more strips and chunks than blocks");
 
-// acc[p] = the fused multiply-add chain over taps k = 0 .. K-1 of
-// x(p + k) * w[k], for kBR consecutive outputs p: the taps ascending from
-// +0 exactly as the one-output loop, with the inputs of a chunk of kBR taps
-// held in registers (each loaded once for the kBR outputs). `at(i)` may be
-// asked for up to 2 kBR - 1 inputs beyond the last one used.
-template <class At>
-__device__ __forceinline__ void chain_r(float (&acc)[kBR], const float* w, int K, At at) {
-  float win[2 * kBR];
+// acc[p] = the chain over taps k = 0 .. K-1 of x(p + k) * w[k] for 8
+// consecutive outputs of two lines, taps ascending from +0. `load8(b, v)` gives
+// the inputs 8 b .. 8 b + 7, called with b = 0, 1, .. in turn, up to 7 inputs
+// past the last one used.
+template <class Load8>
+__device__ __forceinline__ void chain8(f2 (&acc)[8], const f2* w, int K, Load8 load8) {
+  f2 lo[8], hi[8];
 #pragma unroll
-  for (int j = 0; j < kBR; ++j) win[j] = at(j);
-  int k0 = 0;
-  for (; k0 + kBR <= K; k0 += kBR) {
+  for (int p = 0; p < 8; ++p) acc[p] = 0ull;
+  auto block = [&](const f2(&u)[8], const f2(&v)[8], const f2* wk) {
 #pragma unroll
-    for (int j = 0; j < kBR; ++j) win[kBR + j] = at(k0 + kBR + j);
+    for (int j = 0; j < 8; j += 2) {
+      const ulonglong2 w2 = *reinterpret_cast<const ulonglong2*>(wk + j);
 #pragma unroll
-    for (int j = 0; j < kBR; ++j) {
-      const float t = w[k0 + j];
+      for (int p = 0; p < 8; ++p) acc[p] = fma2(p + j < 8 ? u[p + j] : v[p + j - 8], w2.x, acc[p]);
 #pragma unroll
-      for (int p = 0; p < kBR; ++p) acc[p] = fmaf(win[p + j], t, acc[p]);
+      for (int p = 0; p < 8; ++p)
+        acc[p] = fma2(p + j + 1 < 8 ? u[p + j + 1] : v[p + j - 7], w2.y, acc[p]);
     }
-#pragma unroll
-    for (int j = 0; j < kBR; ++j) win[j] = win[kBR + j];
+  };
+  load8(lo);
+  int k = 0;
+  for (; k + 16 <= K; k += 16) {
+    load8(hi);
+    block(lo, hi, w + k);
+    load8(lo);
+    block(hi, lo, w + k + 8);
   }
-  if (k0 < K) {
+  if (k + 8 <= K) {
+    load8(hi);
+    block(lo, hi, w + k);
+    k += 8;
 #pragma unroll
-    for (int j = 0; j < kBR; ++j) win[kBR + j] = at(k0 + kBR + j);
+    for (int j = 0; j < 8; ++j) lo[j] = hi[j];
+  }
+  if (k < K) {  // 1 to 7 taps more
+    load8(hi);
 #pragma unroll
-    for (int j = 0; j < kBR; ++j) {
-      if (k0 + j < K) {
-        const float t = w[k0 + j];
+    for (int j = 0; j < 7; ++j)
+      if (k + j < K) {
+        const f2 wj = w[k + j];
 #pragma unroll
-        for (int p = 0; p < kBR; ++p) acc[p] = fmaf(win[p + j], t, acc[p]);
+        for (int p = 0; p < 8; ++p) acc[p] = fma2(p + j < 8 ? lo[p + j] : hi[p + j - 8], wj, acc[p]);
       }
-    }
   }
 }
 
-__global__ void __launch_bounds__(kBThreads, 3) k_batch_gray_gauss_sobel(const BatchArgs a) {
-  extern __shared__ float smf[];
-  __shared__ CimxBatchTile s_t;                    // this block's tile
-  __shared__ float s_w[kBMaxTaps];                 // this tile's taps
-  __shared__ int s_ci[kBT + 2], s_cj[kBT + 2];     // source row / column of each T row, S column
-  __shared__ int s_yc[kBG], s_xc[kBG];             // group of 8 with consecutive sources
-  const int tid = threadIdx.x;
-  // sizes for the batch's largest radius. Area A: two strip buffers of the
-  // gray region (kCW columns, kSlack spare rows for the register-blocked
-  // chains' reads past the last row), later S. Area B: T (odd row stride,
-  // so that lanes on consecutive rows read different banks).
-  const int gcs = kBT + 3 + 2 * a.max_r;
-  const int gsr = kBT + 2 + 2 * a.max_r + kSlack;
-  float* const Gb0 = smf;
-  float* const Gb1 = smf + gsr * kCW;
-  float* const T = smf + batch_area_a(a.max_r);
-  float* const S = smf;
+// one strip of one chunk of a tile
+struct BatchItem {
+  int tile, x0, xw, y0, rows;  // tile < 0: nothing to do
+};
 
-  for (long long g = blockIdx.x; g < a.nblocks; g += gridDim.x) {
-    if (tid < 32) {
-      // the last tile whose first block <= g, found by the first warp: each
-      // round probes 32 evenly spaced tiles of (lo, hi] and keeps the span
-      // between the last probe <= g and the next one (three rounds for
-      // 4096 tiles)
-      int lo = 0, hi = a.ntiles - 1;
-      while (hi > lo) {
-        const int step = (hi - lo + 31) / 32;
-        const int cand = lo + 1 + tid * step;
-        const bool le = cand <= hi && a.tiles[cand].first_block <= g;
-        const int nle = __popc(__ballot_sync(0xffffffffu, le));
-        if (nle == 0) {
-          hi = lo;
-        } else {
-          lo += 1 + (nle - 1) * step;
-          hi = min(hi, lo + step - 1);
-        }
-      }
-      if (tid == 0) s_t = a.tiles[lo];
+// The item of block index g. A tile's items take the first of its block
+// indexes, the others have none.
+__device__ __forceinline__ BatchItem find_item(const BatchArgs& a, long long g, int lane) {
+  // the last tile whose first block <= g, found by a warp: each round probes 32
+  // evenly spaced tiles of (lo, hi] and keeps the span between the last probe
+  // <= g and the next one (three rounds for 4096 tiles)
+  int lo = 0, hi = a.ntiles - 1;
+  while (hi > lo) {
+    const int step = (hi - lo + 31) / 32;
+    const int cand = lo + 1 + lane * step;
+    const bool le = cand <= hi && a.tiles[cand].first_block <= g;
+    const int nle = __popc(__ballot_sync(0xffffffffu, le));
+    if (nle == 0) {
+      hi = lo;
+    } else {
+      lo += 1 + (nle - 1) * step;
+      hi = min(hi, lo + step - 1);
     }
-    __syncthreads();
-    const CimxBatchTile& t = s_t;
-    const int H = t.height, W = t.width;
+  }
+  BatchItem it{-1, 0, 0, 0, 0};
+  const CimxBatchTile& t = a.tiles[lo];
+  const int K = t.ntaps, H = t.height, W = t.width;
+  const long long j = g - t.first_block;
+  // a block index outside the tile (inconsistent table) is skipped
+  if (j < 0 || K < 1 || K / 2 > a.max_r || H < 1 || W < 1) return it;
+  const int r = K / 2;
+  const int wmax = kBCols - 2 - 2 * r;
+  const int nx = (W + wmax - 1) / wmax, ny = (H + kBRows - 1) / kBRows;
+  if (j >= static_cast<long long>(nx) * ny) return it;
+  const int xw = (W + nx - 1) / nx;
+  const int rows = ((H + ny - 1) / ny + 2 + kBG - 1) / kBG * kBG - 2;
+  it.x0 = static_cast<int>(j % nx) * xw;
+  it.y0 = static_cast<int>(j / nx) * rows;
+  it.xw = min(xw, W - it.x0);
+  it.rows = min(rows, H - it.y0);
+  if (it.xw > 0 && it.rows > 0) it.tile = lo;
+  return it;
+}
+
+// MID: the edge taps have a middle one
+template <bool MID>
+__global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const BatchArgs a) {
+  extern __shared__ __align__(16) unsigned char sm_batch[];
+  __shared__ BatchItem s_item[kBThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  {
+    // one block index per warp, the CTA's indexes a grid apart: those of one
+    // tile's items, which lie together, go to different CTAs
+    const long long g = blockIdx.x + static_cast<long long>(warp) * gridDim.x;
+    BatchItem it{-1, 0, 0, 0, 0};
+    if (g < a.nblocks) it = find_item(a, g, lane);
+    if (lane == 0) s_item[warp] = it;
+  }
+  __syncthreads();
+  f2* const taps = reinterpret_cast<f2*>(sm_batch);
+  float* const ring = reinterpret_cast<float*>(sm_batch + kTapBytes);
+
+  for (int n = 0; n < kBThreads / 32; ++n) {
+    const BatchItem it = s_item[n];
+    if (it.tile < 0) continue;  // the same for every thread
+    const CimxBatchTile& t = a.tiles[it.tile];
+    const int H = t.height, W = t.width, K = t.ntaps, r = K / 2;
     // row pitches: a tile may be a region of a larger slide (0 = packed)
     const long long in_pitch = t.rgb_pitch > 0 ? t.rgb_pitch : 3LL * W;
     const long long out_pitch = t.out_pitch > 0 ? t.out_pitch : W;
-    const int nbx = (W + kBT - 1) / kBT;
-    const long long j = g - t.first_block;
-    // a block index outside the tile (inconsistent table) is skipped; the
-    // test is uniform across the CTA, so every barrier below is still met
-    const bool valid = j >= 0 && j < static_cast<long long>(nbx) * ((H + kBT - 1) / kBT) &&
-                       t.ntaps >= 1 && t.ntaps / 2 <= a.max_r;
-    if (!valid) {
-      __syncthreads();
-      continue;
-    }
-    const int y0 = static_cast<int>(j / nbx) * kBT, x0 = static_cast<int>(j % nbx) * kBT;
-    const int K = t.ntaps, r = K / 2;
-    const float* w = a.taps + t.taps_offset;
-    const int GR = kBT + 2 + 2 * r, GC = kBT + 2 + 2 * r;
+    const uint8_t* const rgb = t.rgb;
+    float* const out = t.out;
+    const int R = ring_rows(K), SP = s_pitch(K);
+    unsigned char* const T = reinterpret_cast<unsigned char*>(ring + R * kBCols);
+    f2* const S = reinterpret_cast<f2*>(T + kTBytes);
+    // the smoothed row s of the walk is row ys + s of the tile, and the
+    // smoothed column c is column x0 - 1 + c; gray row j is row ys - r + j,
+    // gray column c is column x0 - 1 - r + c (both 'nearest')
+    const int ys = it.y0 - 1;
+    const int ns = it.xw + 2;           // smoothed columns
+    const int need = ns + 2 * r;        // staged columns in use
+    const int groups = (it.rows + 2 + kBG - 1) / kBG;
 
-    // 0. the tile's taps, and the source row / column (in the gray region)
-    //    of every smoothed row / column the edge passes read: 'reflect'
-    //    around the tile, kept inside the region
-    for (int k = tid; k < K; k += kBThreads) s_w[k] = w[k];
-    for (int i = tid; i < kBT + 2; i += kBThreads) {
-      int ci = map_coord32(y0 - 1 + i, H, CIMX_MODE_REFLECT) - (y0 - 1 - r);
-      s_ci[i] = ci < r ? r : (ci > GR - 1 - r ? GR - 1 - r : ci);
-      int cj = map_coord32(x0 - 1 + i, W, CIMX_MODE_REFLECT) - (x0 - 1 - r);
-      s_cj[i] = cj < r ? r : (cj > GC - 1 - r ? GC - 1 - r : cj);
-    }
-    __syncthreads();
-    if (tid < 2 * kBG) {
-      const int q = tid % kBG, i0 = q * kBR;
-      const int* src = tid < kBG ? s_ci : s_cj;
-      int ok = i0 + kBR <= kBT + 2;
-      for (int p = 1; ok && p < kBR; ++p) ok = src[i0 + p] == src[i0] + p;
-      (tid < kBG ? s_yc : s_xc)[q] = ok;
+    for (int k = tid; k < K; k += kBThreads) {
+      const float w = a.taps[t.taps_offset + k];
+      taps[k] = pack2(w, w);
     }
 
-    // 1-2. the gray region (rows y0-1-r .., columns x0-1-r .., 'nearest'
-    //    borders) and the gaussian along y, in strips of kCW region columns
-    //    through two buffers: while the y pass runs on strip s, the words of
-    //    strip s + 1 are in flight. Gray: a thread takes groups of 4
-    //    consecutive pixels of a row; where they lie inside the row, their
-    //    12 bytes come from three or four aligned 32-bit words (each word
-    //    holds at least one of the 12 bytes, so it lies in the tile's
-    //    allocation), at the tile's borders pixel by pixel. The y pass: T
-    //    row tr is the smoothed row refl(y0 - 1 + tr) (rows outside the tile
-    //    only feed outputs that are not stored); a thread takes 8
-    //    consecutive T rows of one column, one by one where their source
-    //    rows are not consecutive (tile borders).
-    const int ng = GR * kCG;       // 4-pixel groups of one strip
-    const int xb = x0 - 1 - r;     // source column of region column 0
-    const int nstrips = (GC + kCW - 1) / kCW;
-    uint32_t wv[kGB][4];
-    unsigned shv[kGB];
-    bool fast[kGB];
-    auto gray_load = [&](int st, int i0) {
+    // gray: 4 consecutive pixels of every fourth row. Inside the tile's row
+    // their 12 bytes come from three or four aligned words (each holds at least
+    // one of the bytes, so it lies in the tile's allocation); at its ends byte
+    // by byte.
+    const int gc = (tid & 63) * 4, grow = tid >> 6;
+    const int xs = it.x0 - 1 - r + gc;
+    const bool gon = gc < need;
+    const bool words = xs >= 0 && xs + 3 < W;
+    uint32_t wv[4][4];
+    unsigned shv[4];
+    auto gray_load = [&](int j0) {
+      if (!gon) return;
 #pragma unroll
-      for (int u = 0; u < kGB; ++u) {
-        const int idx = i0 + u * kBThreads;
-        const int gr = idx / kCG, c0 = st * kCW + (idx - gr * kCG) * 4;
-        const int xs = xb + c0;
-        fast[u] = idx < ng && c0 + 3 < GC && xs >= 0 && xs + 3 < W;
-        shv[u] = 0;
-        wv[u][0] = wv[u][1] = wv[u][2] = wv[u][3] = 0u;
-        if (fast[u]) {
-          const uint8_t* px = t.rgb + static_cast<long long>(nearest_idx(y0 - 1 - r + gr, H)) * in_pitch + 3LL * xs;
-          const uintptr_t pa = reinterpret_cast<uintptr_t>(px);
+      for (int u = 0; u < 4; ++u) {
+        const int y = min(max(ys - r + j0 + grow + 4 * u, 0), H - 1);
+        const uint8_t* row = rgb + y * in_pitch;
+        if (words) {
+          const uintptr_t pa = reinterpret_cast<uintptr_t>(row + 3LL * xs);
           const uint32_t* wp = reinterpret_cast<const uint32_t*>(pa & ~static_cast<uintptr_t>(3));
           shv[u] = static_cast<unsigned>(pa & 3) * 8u;
           wv[u][0] = __ldg(wp);
           wv[u][1] = __ldg(wp + 1);
           wv[u][2] = __ldg(wp + 2);
+          wv[u][3] = 0u;
           if (shv[u]) wv[u][3] = __ldg(wp + 3);
-        }
-      }
-    };
-    auto gray_store = [&](int st, int i0) {
-      float* Gs = (st & 1) ? Gb1 : Gb0;
-#pragma unroll
-      for (int u = 0; u < kGB; ++u) {
-        const int idx = i0 + u * kBThreads;
-        if (idx >= ng) break;
-        const int gr = idx / kCG, cl = (idx - gr * kCG) * 4, c0 = st * kCW + cl;
-        if (c0 >= GC) continue;
-        float* dst = Gs + gr * kCW + cl;
-        if (fast[u]) {
-          const unsigned sh = shv[u];
-          const uint32_t v0 = __funnelshift_r(wv[u][0], wv[u][1], sh);
-          const uint32_t v1 = __funnelshift_r(wv[u][1], wv[u][2], sh);
-          const uint32_t v2 = __funnelshift_r(wv[u][2], wv[u][3], sh);
-          // one 16-byte store: strip rows are 28 floats and groups start at
-          // multiples of 4, so dst is 16-byte aligned
-          *reinterpret_cast<float4*>(dst) = make_float4(
-              luma_f64(chan(v0 & 255u), chan((v0 >> 8) & 255u), chan((v0 >> 16) & 255u)),
-              luma_f64(chan(v0 >> 24), chan(v1 & 255u), chan((v1 >> 8) & 255u)),
-              luma_f64(chan((v1 >> 16) & 255u), chan(v1 >> 24), chan(v2 & 255u)),
-              luma_f64(chan((v2 >> 8) & 255u), chan((v2 >> 16) & 255u), chan(v2 >> 24)));
         } else {
-          const uint8_t* row = t.rgb + static_cast<long long>(nearest_idx(y0 - 1 - r + gr, H)) * in_pitch;
-          const int xs = xb + c0;
-          for (int p = 0; p < 4 && c0 + p < GC; ++p) {
+          shv[u] = 0;
+          wv[u][0] = wv[u][1] = wv[u][2] = wv[u][3] = 0u;
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
             const uint8_t* px = row + 3LL * nearest_idx(xs + p, W);
-            dst[p] = luma_f64(chan(px[0]), chan(px[1]), chan(px[2]));
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+              wv[u][(3 * p + c) / 4] |= static_cast<uint32_t>(__ldg(px + c)) << ((3 * p + c) % 4 * 8);
           }
         }
       }
     };
-    auto ypass = [&](int st) {
-      const float* Gs = (st & 1) ? Gb1 : Gb0;
-      for (int idx = tid; idx < kBG * kCW; idx += kBThreads) {
-        const int q = idx / kCW, cl = idx - q * kCW, c = st * kCW + cl;
-        if (c >= GC) continue;
-        const int tr0 = q * kBR, nr = min(kBR, kBT + 2 - tr0);
-        if (s_yc[q]) {
-          float acc[kBR];
+    auto gray_store = [&](int slot) {  // ring slot of the first of the kBG rows (a multiple of 8)
+      if (!gon) return;
 #pragma unroll
-          for (int p = 0; p < kBR; ++p) acc[p] = 0.f;
-          const float* col = Gs + (s_ci[tr0] - r) * kCW + cl;
-          chain_r(acc, s_w, K, [&](int i) { return col[i * kCW]; });
-#pragma unroll
-          for (int p = 0; p < kBR; ++p) T[(tr0 + p) * gcs + c] = acc[p];
-        } else {
-          for (int p = 0; p < nr; ++p) {
-            const float* col = Gs + (s_ci[tr0 + p] - r) * kCW + cl;
-            float acc = 0.f;
-            for (int k = 0; k < K; ++k) acc = fmaf(col[k * kCW], s_w[k], acc);
-            T[(tr0 + p) * gcs + c] = acc;
-          }
-        }
+      for (int u = 0; u < 4; ++u) {
+        const uint32_t v0 = __funnelshift_r(wv[u][0], wv[u][1], shv[u]);
+        const uint32_t v1 = __funnelshift_r(wv[u][1], wv[u][2], shv[u]);
+        const uint32_t v2 = __funnelshift_r(wv[u][2], wv[u][3], shv[u]);
+        int q = slot + grow + 4 * u;
+        if (q >= R) q -= R;
+        *reinterpret_cast<float4*>(ring + q * kBCols + gc) = make_float4(
+            luma(v0 & 255u, (v0 >> 8) & 255u, (v0 >> 16) & 255u),
+            luma(v0 >> 24, v1 & 255u, (v1 >> 8) & 255u),
+            luma((v1 >> 16) & 255u, v1 >> 24, v2 & 255u),
+            luma((v2 >> 8) & 255u, (v2 >> 16) & 255u, v2 >> 24));
       }
     };
-    for (int i0 = tid; i0 < ng; i0 += kGB * kBThreads) {
-      gray_load(0, i0);
-      gray_store(0, i0);
+
+    // the first group's rows: R = K - 1 + kBG rounded up, a multiple of 8; the
+    // last fill may wrap on to the ring's start when R is not a multiple of
+    // kBG, so it fills only what is left
+    for (int j = 0; j + kBG <= R; j += kBG) {
+      gray_load(j);
+      gray_store(j);
+    }
+    if (R % kBG) {  // 8 rows left, filled together with the 8 before them
+      gray_load(R - kBG);
+      gray_store(R - kBG);
     }
     __syncthreads();
-    for (int st = 0; st < nstrips; ++st) {
-      const bool next = st + 1 < nstrips;  // the same for every thread
-      if (next) gray_load(st + 1, tid);
-      ypass(st);
-      if (next) {
-        gray_store(st + 1, tid);
-        for (int i0 = tid + kGB * kBThreads; i0 < ng; i0 += kGB * kBThreads) {
-          gray_load(st + 1, i0);
-          gray_store(st + 1, i0);
+
+    int base = 0;           // ring slot of the group's first gray row
+    for (int g = 0; g < groups; ++g) {
+      const bool more = g + 1 < groups;
+      // the kBG rows after the ring's last one
+      if (more) gray_load(R + g * kBG);
+      {
+        // y chains: column pair p, rows 8 q .. 8 q + 7 of the group
+        const int p = tid & 127, q = tid >> 7;
+        if (2 * p < need) {
+          int slot = base + 8 * q;
+          if (slot >= R) slot -= R;
+          const float* col = ring + 2 * p;
+          f2 acc[8];
+          chain8(acc, taps, K, [&](f2(&v)[8]) {
+            const float* at = col + slot * kBCols;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const f2*>(at + j * kBCols);
+            slot += 8;
+            if (slot == R) slot = 0;
+          });
+          unsigned char* put = T + 4 * q * kTPitch + 16 * p;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<float4*>(put + i * kTPitch) = make_float4(
+                lo2(acc[2 * i]), lo2(acc[2 * i + 1]), hi2(acc[2 * i]), hi2(acc[2 * i + 1]));
         }
       }
       __syncthreads();
-    }
-
-    // 3. gaussian along x: S(sr, sc) is the smoothed value at
-    //    (refl(y0 - 1 + sr), refl(x0 - 1 + sc)); a thread takes 8
-    //    consecutive columns of one row (lanes on consecutive rows)
-    for (int idx = tid; idx < kBG * (kBT + 2); idx += kBThreads) {
-      const int q = idx / (kBT + 2), sr = idx - q * (kBT + 2);
-      const int sc0 = q * kBR, nc = min(kBR, kBT + 2 - sc0);
-      if (s_xc[q]) {
-        float acc[kBR];
+      if (more) gray_store(base);
+      base += kBG;
+      if (base >= R) base -= R;
+      {
+        // x chains: row pair rp, smoothed columns c0 .. c0 + 7
+        const int rp = tid & 7, c0 = (tid >> 3) * 8;
+        if (c0 < ns) {
+          const unsigned char* at = T + rp * kTPitch + c0 * 8;
+          f2 acc[8];
+          chain8(acc, taps, K, [&](f2(&v)[8]) {
 #pragma unroll
-        for (int p = 0; p < kBR; ++p) acc[p] = 0.f;
-        const float* row = T + sr * gcs + (s_cj[sc0] - r);
-        chain_r(acc, s_w, K, [&](int i) { return row[i]; });
+            for (int j = 0; j < 8; j += 2) {
+              const ulonglong2 e = *reinterpret_cast<const ulonglong2*>(at + j * 8);
+              v[j] = e.x;
+              v[j + 1] = e.y;
+            }
+            at += 64;
+          });
+          // 'reflect' around the tile: the first row (here), column and the last
+          // column once more; the last row where the edges read it
+          if (g == 0 && rp == 0 && ys < 0) {
 #pragma unroll
-        for (int p = 0; p < kBR; ++p) S[sr * kSS + sc0 + p] = acc[p];
-      } else {
-        for (int p = 0; p < nc; ++p) {
-          const float* row = T + sr * gcs + (s_cj[sc0 + p] - r);
-          float acc = 0.f;
-          for (int k = 0; k < K; ++k) acc = fmaf(row[k], s_w[k], acc);
-          S[sr * kSS + sc0 + p] = acc;
+            for (int e = 0; e < 8; ++e) acc[e] = pack2(hi2(acc[e]), hi2(acc[e]));
+          }
+          const int x = it.x0 - 1 + c0;
+          f2* row = S + ((g * (kBG / 2) + rp) % (kBSRows / 2)) * SP + c0;
+          if (x >= 0 && x + 7 < W - 1) {
+#pragma unroll
+            for (int e = 0; e < 8; e += 2)
+              *reinterpret_cast<ulonglong2*>(row + e) = make_ulonglong2(acc[e], acc[e + 1]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              if (x + e >= 0 && x + e < W && c0 + e < ns) {
+                row[e] = acc[e];
+                if (x + e == 0) row[e - 1] = acc[e];
+                if (x + e == W - 1) row[e + 1] = acc[e];
+              }
+          }
+        }
+      }
+      __syncthreads();
+      {
+        // edges (E0 along y, E1 along x), smoothing and magnitude of output
+        // rows s = 16 g - 1 + 4 rq + i of the walk, from the row pairs s - 1 ..
+        // s + 4. Each value is the same chain as a separate pass over stored E0
+        // and E1 would compute, two rows at a time.
+        const int rq = warp & 3;
+        const int s0 = g * kBG - 1 + 4 * rq;
+        const f2* pair[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+          pair[i] = S + (max(g * (kBG / 2) - 1 + 2 * rq + i, 0) % (kBSRows / 2)) * SP;
+        const int below = H - (ys + s0 - 1);  // index of the row below the last one
+        const bool bottom = below < 6;
+        auto edge2 = [&](f2 u, f2 v, f2 w) {
+          f2 e = fma2(u, pack2(a.edge[0], a.edge[0]), 0ull);
+          if (MID) e = fma2(v, pack2(a.edge[1], a.edge[1]), e);
+          return fma2(w, pack2(a.edge[2], a.edge[2]), e);
+        };
+        auto smooth2 = [&](f2 u, f2 v, f2 w) {
+          return fma2(w, pack2(a.smooth[2], a.smooth[2]),
+                      fma2(v, pack2(a.smooth[1], a.smooth[1]),
+                           fma2(u, pack2(a.smooth[0], a.smooth[0]), 0ull)));
+        };
+        for (int c = (warp >> 2) * 32 + lane; c < it.xw; c += 64) {
+          f2 v[3][3], e1[3];
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[i][k] = pair[i][c + k];
+          if (bottom) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+              for (int k = 0; k < 3; ++k) {
+                if (i > 0 && below == 2 * i) v[i][k] = pack2(hi2(v[i - 1][k]), hi2(v[i][k]));
+                if (below == 2 * i + 1) v[i][k] = pack2(lo2(v[i][k]), lo2(v[i][k]));
+              }
+          }
+#pragma unroll
+          for (int i = 0; i < 3; ++i) e1[i] = edge2(v[i][0], v[i][1], v[i][2]);
+          float* o = out + (ys + s0) * out_pitch + it.x0 + c;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            f2 e0[3];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+              e0[k] = edge2(v[i][k], pack2(hi2(v[i][k]), lo2(v[i + 1][k])), v[i + 1][k]);
+            const f2 d0 = smooth2(e0[0], e0[1], e0[2]);
+            const f2 d1 = smooth2(e1[i], pack2(hi2(e1[i]), lo2(e1[i + 1])), e1[i + 1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const float p = h ? hi2(d0) : lo2(d0), q = h ? hi2(d1) : lo2(d1);
+              const int s = s0 + 2 * i + h;
+              if (s >= 1 && s <= it.rows)
+                o[(2 * i + h) * out_pitch] = sqrtf(__fadd_rn(__fmul_rn(p, p), __fmul_rn(q, q)));
+            }
+          }
         }
       }
     }
-    __syncthreads();
-
-    // 4-5. edge passes (E0 along y, E1 along x), smoothing passes and the
-    //    magnitude, per 4 consecutive outputs of a row: every E0 and E1
-    //    value they read comes from the 3 x 6 window of S at (y, x), kept in
-    //    registers; each value is the same chain as a separate pass over a
-    //    stored E0 / E1 would compute. Lanes take consecutive rows (S's odd
-    //    row stride: conflict-free).
-    for (int it = tid; it < kBT * (kBT / 4); it += kBThreads) {
-      const int y = it % kBT, x = (it / kBT) * 4;
-      if (y0 + y >= H || x0 + x >= W) continue;
-      float sw[3][6];
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int c = 0; c < 6; ++c) sw[i][c] = S[(y + i) * kSS + x + c];
-      float e0[6], e1[3][4];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        float acc = 0.f;
-        acc = fmaf(sw[0][c], a.edge[0], acc);
-        acc = fmaf(sw[1][c], a.edge[1], acc);
-        acc = fmaf(sw[2][c], a.edge[2], acc);
-        e0[c] = acc;
-      }
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float acc = 0.f;
-          acc = fmaf(sw[i][c], a.edge[0], acc);
-          acc = fmaf(sw[i][c + 1], a.edge[1], acc);
-          acc = fmaf(sw[i][c + 2], a.edge[2], acc);
-          e1[i][c] = acc;
-        }
-      float* orow = t.out + static_cast<long long>(y0 + y) * out_pitch + x0 + x;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float d0 = 0.f;
-        d0 = fmaf(e0[c], a.smooth[0], d0);
-        d0 = fmaf(e0[c + 1], a.smooth[1], d0);
-        d0 = fmaf(e0[c + 2], a.smooth[2], d0);
-        float d1 = 0.f;
-        d1 = fmaf(e1[0][c], a.smooth[0], d1);
-        d1 = fmaf(e1[1][c], a.smooth[1], d1);
-        d1 = fmaf(e1[2][c], a.smooth[2], d1);
-        const float m = __fadd_rn(__fmul_rn(d0, d0), __fmul_rn(d1, d1));
-        if (x0 + x + c < W) orow[c] = sqrtf(m);
-      }
-    }
-    __syncthreads();  // shared buffers are reused by the next block
+    __syncthreads();  // the next item's ring may lie over this one's S
   }
 }
 
@@ -419,30 +480,24 @@ extern "C" int cimx_batch_gray_gauss_sobel(const CimxBatchTile* tiles, int ntile
     a.edge[k] = edge_taps[k];
     a.smooth[k] = smooth_taps[k];
   }
-  const size_t smem = sizeof(float) * (static_cast<size_t>(batch_area_a(a.max_r)) +
-                                       static_cast<size_t>(batch_area_b(a.max_r)));
-  // the kernel also holds about 1.2 KB of static shared memory (taps, the
-  // row / column tables); the sum stays under the 227 KB per CTA
+  const size_t smem = batch_smem(max_taps);
   constexpr int kDynLimit = 223 * 1024;
-  if (smem > static_cast<size_t>(kDynLimit)) return fail(CIMX_E_INVALID, "batch: taps too long");
+  auto* kern = edge_taps[1] != 0.f ? k_batch_gray_gauss_sobel<true> : k_batch_gray_gauss_sobel<false>;
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    attr_err = cudaFuncSetAttribute(k_batch_gray_gauss_sobel,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, kDynLimit);
+    for (auto* k : {k_batch_gray_gauss_sobel<true>, k_batch_gray_gauss_sobel<false>}) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynLimit);
+      if (e != cudaSuccess) attr_err = e;
+    }
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "batch: shared memory attribute");
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // resident CTAs per SM: three while the shared memory allows (largest
-  // radius up to about 38), two beyond; the grid walks the block list with
-  // a stride
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_gray_gauss_sobel, kBThreads,
-                                                    smem) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  const long long grid = std::min<long long>(nblocks, static_cast<long long>(per_sm) * sms);
-  k_batch_gray_gauss_sobel<<<(unsigned)grid, kBThreads, smem, static_cast<cudaStream_t>(stream)>>>(a);
+  // a CTA takes one block index per warp; those without an item cost it the
+  // lookup alone
+  constexpr int kPer = kBThreads / 32;
+  const long long grid = (nblocks + kPer - 1) / kPer;
+  if (grid > 0x7fffffffLL) return fail(CIMX_E_INVALID, "batch: too many blocks");
+  kern<<<(unsigned)grid, kBThreads, smem, static_cast<cudaStream_t>(stream)>>>(a);
   return cuda_fail(cudaGetLastError(), "batch launch");
 }

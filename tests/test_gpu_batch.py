@@ -145,3 +145,22 @@ def test_region_stream_rejects_bad_input(cuda):
         batch.RegionStream([np.zeros((4, 4, 3), np.float32)], [1.0])
     with pytest.raises(ValueError):
         batch.RegionStream.from_regions(np.zeros((10, 10, 3), np.uint8), [(5, 5, 6, 2)], [1.0])
+
+
+# strips end at 254 - 2r output columns and chunks at 254 rows
+@pytest.mark.parametrize("sigma", [0.1, 0.5, 2.0, 3.7, 8.0, 16.0])
+def test_batch_strip_edges(cuda, sigma):
+    from cucim_b200 import batch
+
+    wmax = 254 - 2 * int(4 * sigma + 0.5)
+    shapes = [(14, wmax), (15, wmax + 1), (254, 9), (255, wmax - 1), (508, 2 * wmax + 1), (2, 1),
+              (1, 7), (31, 2 * wmax)]
+    tiles = _tiles(shapes, 8)
+    # one more as a region of a larger image, off the word boundaries
+    tiles.append(_tiles([(300, 331)], 9)[0][5:290, 3:3 + 277])
+    b = batch.TileBatch(tiles, [sigma] * len(tiles))
+    got = b.run()
+    ref = batch.gray_gauss_sobel_per_tile([t.contiguous() for t in tiles], [sigma] * len(tiles))
+    torch.cuda.synchronize()
+    for g, r, t in zip(got, ref, tiles):
+        assert torch.equal(g, r), (tuple(t.shape), (g - r).abs().max().item())
