@@ -29,7 +29,7 @@ bool fast_pair(int t, int d) {
 struct Trimmed {
   int K = 0, anchor = 0;
   bool interior_zero = false;
-  float w[kSlabMaxK];
+  float w[kLongMaxK];
 };
 
 // Taps rounded to float32; with the elementwise-kernel rule, zero taps at
@@ -69,6 +69,8 @@ int launch_columns(const PassDesc& d, const Trimmed& t, int tin, const void* in,
                    void* out, cudaStream_t st) {
   if (d.outer * d.L * d.inner == 0) return CIMX_OK;
   const bool skip = d.skip_zero && t.interior_zero;
+  if (tin == DT_F32 && tout == DT_F32 && ring_takes(d.L, t.K))
+    return launch_ring_f32(d, t.w, t.K, t.anchor, skip, in, out, st);
   switch (tin) {
     case DT_F32: return launch_columns_f32(d, t.w, t.K, t.anchor, skip, in, tout, out, st);
     case DT_U16: return launch_columns_u16(d, t.w, t.K, t.anchor, skip, in, tout, out, st);
@@ -200,10 +202,11 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
     for (int i = 0; i < npasses; ++i) {
       const int tin = i == 0 ? in->dtype : D;
       Step s{kGeneric, i, -1};
-      if (nd >= 2 && fast_pair(tin, D) && trim(ds[i], kSlabMaxK, tr[i])) {
+      const bool f32 = tin == DT_F32 && D == DT_F32;
+      if (nd >= 2 && fast_pair(tin, D) && trim(ds[i], f32 ? kLongMaxK : kSlabMaxK, tr[i])) {
         if (ds[i].axis == nd - 1) {
           if (n / std::max<int64_t>(1, in->shape[nd - 1]) >= kStripMinRows) s = {kStrip, -1, i};
-        } else if (ds[i].axis == nd - 2 && i + 1 < npasses &&
+        } else if (ds[i].axis == nd - 2 && i + 1 < npasses && tr[i].K <= kSlabMaxK &&
                    trim(ds[i + 1], kSlabMaxK, tr[i + 1]) &&
                    (fuse_all || strip_fuses(dtype_size(tin), ds[i], tr[i], ds[i + 1], tr[i + 1]))) {
           s = {kStrip, i, i + 1};

@@ -13,14 +13,15 @@ namespace cimx {
 // then runs the passes one launch at a time.
 constexpr int CIMX_FUSED_DECLINED = 1;
 
-constexpr int kSlabMaxK = 65;  // longest pass the strip and column kernels take
+constexpr int kSlabMaxK = 65;   // longest pass the strip and column kernels take
+constexpr int kLongMaxK = 129;  // the same for a float32 pass of its own
 
 // One pass of the strip and volume kernels (float32 weights, already trimmed).
 struct SlabPass {
   int K, anchor, mode;
   double cval;
   int cval_as_input, dt, skip, pad;
-  float w[kSlabMaxK];
+  float w[kLongMaxK];
 };
 
 struct SlabArgs {
@@ -67,6 +68,15 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
 // elementwise copy with conversion (used when a filter has no passes)
 int launch_copy_cast(const void* in, int tin, void* out, int tout, int64_t n,
                      cudaStream_t stream);
+
+// Whether a float32 pass along a strided axis takes the ring kernel
+// (cimx_ring.cuh) rather than k_columns: axis 0 of 8192^2 / of 256^3, us, ring
+// against k_columns: 21 taps 104 / 39 against 115 / 37, 25 taps 108 / 38 against
+// 124 / 42, 41 taps 126 / 39 against 160 / 50, 65 taps 181 / 56 against 213 / 73.
+// A step is 64 rows: shorter axes leave its warps idle.
+inline bool ring_takes(int64_t L, int K) { return K > kSlabMaxK || (K >= 22 && L >= 48); }
+int launch_ring_f32(const PassDesc& d, const float* w, int K, int anchor, bool skip,
+                    const void* in, void* out, cudaStream_t st);
 
 // single-launch 3-D filter, by input dtype; equal K in {3, 5} on every axis
 int launch_vol_f32(const VolArgs& v, int tout, cudaStream_t st);

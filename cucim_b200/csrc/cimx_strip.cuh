@@ -30,7 +30,8 @@
 // 335; one 2048^2 image, 33 taps 23.7 against 33.0; 256 x 512^2 uint16, 17
 // taps 176 (to float32) and 189 (to uint16) against 278 and 314, and 255 x 511
 // x 509, whose rows the tile kernel could not load, 214 against 813. An x pass
-// alone, 256^3 float32, 17 / 57 taps: 33 / 53 against 65 / 156.
+// alone, 256^3 float32, 17 / 57 taps: 33 / 53 against 65 / 156; 8192^2, 129 taps
+// 293 us (82 % of the FMA rate) against 699 on k_rows (taps in shared memory).
 //
 // Also measured: one column per thread with scalar FMAs, which doubles the
 // warps: 364 instead of 294 us at 128 x 1024^2, 17 taps (twice the shared
@@ -138,12 +139,15 @@ __device__ __forceinline__ uint32_t load_rows(typename Raw<T>::type (&v)[kN], co
   return fill;
 }
 
+constexpr int act_words(int KT) { return (KT + 31) / 32; }
+
 // Tests of the taps of one chain: KT slots, K of them in use. GEN false: K lies
 // in (KT - NP, KT] and only the centre tap may be left out (slot `centre`, the
 // zero of an odd Gaussian derivative). GEN true: a bit per slot. Taps sit in
 // the first K slots (LAST false) or in the last K.
 template <int KT, int NP, bool GEN, bool LAST>
-__device__ __forceinline__ bool tap_on(int k, int K, int centre, const uint32_t (&act)[3]) {
+__device__ __forceinline__ bool tap_on(int k, int K, int centre,
+                                       const uint32_t (&act)[act_words(KT)]) {
   if constexpr (GEN) {
     return (act[k >> 5] >> (k & 31)) & 1u;
   } else {
@@ -159,7 +163,7 @@ __device__ __forceinline__ bool tap_on(int k, int K, int centre, const uint32_t 
 template <int KT, class W>
 struct SlotTaps {
   int K, centre;        // centre: slot of a centre tap that is left out, or -1
-  uint32_t act[3];
+  uint32_t act[act_words(KT)];
   W w[KT];
 };
 
@@ -240,6 +244,7 @@ __device__ __forceinline__ void store_row(D* p, const float (&v)[kP], int left, 
 // per thread, and a spill waits for the loads in flight (float32, 9 taps at
 // three CTAs: 96 bytes spilled, 128 x 1024^2 in 474 us against 238 at two).
 constexpr int kStripThreads = 256;
+constexpr int kLongThreads = 224;  // beyond kSlabMaxK taps: shared memory
 template <class T> constexpr int strip_ctas(int KY) { return KY <= (sizeof(T) == 4 ? 5 : 9) ? 3 : 2; }
 
 template <int KY, int KX>
@@ -562,7 +567,9 @@ int trunc_bounded(const float* w, int K, int mode, double cval, double& bound) {
   return bound < dmax + 1.0;
 }
 
-static_assert(smem_bytes<kSlabMaxK>(kStripThreads) <= 48 * 1024, "no opt-in shared memory");
+static_assert(smem_bytes<kLongMaxK>(kLongThreads) <= 48 * 1024 &&
+                  smem_bytes<kSlabMaxK>(kStripThreads) <= 48 * 1024,
+              "no opt-in shared memory");
 
 template <class T, class D, int KY, int KX, int NP, bool GEN>
 int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
@@ -596,7 +603,7 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
   static int occ[kStripThreads / 32 + 1] = {};  // resident CTAs per SM, by warps
   static std::once_flag once;
   std::call_once(once, [&] {
-    for (int nt = 64; nt <= kStripThreads; nt += 32) {
+    for (int nt = 64; nt <= (KX > kSlabMaxK ? kLongThreads : kStripThreads); nt += 32) {
       int v = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, nt, smem_bytes<KX>(nt)) != cudaSuccess ||
           v < 1)
@@ -614,8 +621,12 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
     // CTA width: the staged columns of all tiles together as few as possible
     int nt = 0;
     long long tiles = 0, best = 0;
-    for (int w = 64; w <= kStripThreads; w += 32) {
-      const int xw = (2 * w - (a.x.K - 1)) / 16 * 16;
+    constexpr int kMost = KX > kSlabMaxK ? kLongThreads : kStripThreads;
+    for (int w = 64; w <= kMost; w += 32) {
+      int xw = (2 * w - (a.x.K - 1)) / 16 * 16;
+      // long filters: four warps of x work, one per scheduler, of the six or
+      // seven that stage (8192^2, 129 taps: 414 us with five)
+      if (KX > kSlabMaxK) xw = std::min(xw, 256);
       if (xw < 16) continue;
       const long long tl = (s.X + xw - 1) / xw;
       long long cost = tl * w;
@@ -695,7 +706,21 @@ int launch_strip_td(const SlabArgs& s, cudaStream_t st) {
   const bool masked = skip_kind(s.py.w, s.py.K, s.py.skip) == 2 ||
                       skip_kind(s.px.w, s.px.K, s.px.skip) == 2;
   if (!s.has_y) {
+    if constexpr (sizeof(T) == 4) {
+      if (masked && K > kSlabMaxK) return launch_strip_k<T, D, 1, kLongMaxK, kLongMaxK, true>(s, st);
+    }
     if (masked) return launch_strip_k<T, D, 1, 65, 65, true>(s, st);
+    if constexpr (sizeof(T) == 4) {
+      if (K > kSlabMaxK) {
+        switch ((kt + 7 - 1) / 8 * 8 + 1) {
+#define CIMX_KT(K_) case K_: return launch_strip_k<T, D, 1, K_, 8, false>(s, st);
+          CIMX_KT(73) CIMX_KT(81) CIMX_KT(89) CIMX_KT(97) CIMX_KT(105) CIMX_KT(113) CIMX_KT(121)
+          CIMX_KT(129)
+#undef CIMX_KT
+          default: return CIMX_FUSED_DECLINED;
+        }
+      }
+    }
     switch (kt) {
       case 5: case 9: return launch_strip_k<T, D, 1, 9, 9, false>(s, st);
 #define CIMX_KT(K_) case K_: return launch_strip_k<T, D, 1, K_, 8, false>(s, st);

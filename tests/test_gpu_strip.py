@@ -138,3 +138,23 @@ def test_long_tail_passes_without_scratch_memory(ndi):
                  "float32")
     finally:
         set_allocator(None, None, None)
+
+
+@pytest.mark.parametrize("K", [22, 25, 26, 57, 66, 73, 74, 97, 128, 129, 130])
+@pytest.mark.parametrize("shape", [(150, 70), (64, 321), (41, 129), (257, 33), (300, 64)])
+def test_long_passes(ndi, K, shape):
+    """Long passes each in a launch of their own (cimx_ring.cuh along a strided
+    axis), around its step of 64 rows, 64 columns and the tap bounds."""
+    x = _data(shape, "float32", K)
+    x[3, 5], x[20, 30], x[40, 11] = np.inf, np.nan, -np.inf
+    for i, kind in enumerate(("plain", "centre", "holes")):
+        w = _taps(K, kind)
+        for mode in MODES[i % 2::2]:
+            for ax in (0, 1):
+                _run(ndi, x, [(ax, w, mode, 0)], "float32", cval=2.5)
+        _run(ndi, x, [(0, w, MODES[i], (K - 1) // 2), (1, w, MODES[4 - i], -(K // 2))],
+             "float32", cval=np.inf if i == 1 else 0.5)
+    flat = _data(shape[0] * shape[1] + 1, "float32", K)  # off the vector boundary
+    xd = torch.as_tensor(flat).cuda()[1:].view(shape)
+    got = ndi.correlate1d(xd, w, axis=0).cpu().numpy()
+    np.testing.assert_array_equal(got, R.correlate1d(flat[1:].reshape(shape), w, 0))
