@@ -184,7 +184,9 @@ __global__ void k_eig22(const F* __restrict__ M00, const F* __restrict__ M01,
 
 // feature/corner.py:566-647 — symmetric 3x3 eigenvalues, float64 inside
 // (Deledalle et al. closed form with the max(.,0) guards). Arguments are the
-// matrix [[a d f] [d b e] [f e c]].
+// matrix [[a d f] [d b e] [f e c]]. Bound: the float64 pipe (half the float32
+// rate). 256^3 float32: 220 us against 331 with three cosines of divided angles;
+// with the vesselness (k_frangi_fused) 355 against 479.
 template <class F>
 __device__ __forceinline__ void eig33(double a, double b, double c, double d, double e, double f,
                                       F& lam1, F& lam2, F& lam3) {
@@ -207,11 +209,16 @@ __device__ __forceinline__ void eig33(double a, double b, double c, double d, do
     phi = atan(sqrt(arg) / x2);
     if (x2 < 0) phi += M_PI;
   }
-  double x1_term = (2.0 / 3.0) * sqrt(x1);
-  double abc = (a + b + c) / 3.0;
-  lam1 = abc - x1_term * cos(phi / 3.0);
-  lam2 = abc + x1_term * cos((phi - M_PI) / 3.0);
-  lam3 = abc + x1_term * cos((phi + M_PI) / 3.0);
+  // cos((phi -+ pi) / 3) = cos(phi / 3) / 2 +- sin(phi / 3) sqrt(3) / 2: one
+  // sine and cosine for the three cosines and their three divisions
+  double sn, cs;
+  sincos(phi * (1.0 / 3.0), &sn, &cs);
+  const double x1_term = (2.0 / 3.0) * sqrt(x1);
+  const double abc = (a + b + c) * (1.0 / 3.0);
+  const double h = 0.5 * cs, q = 0.86602540378443864676 * sn;
+  lam1 = abc - x1_term * cs;
+  lam2 = abc + x1_term * (h + q);
+  lam3 = abc + x1_term * (h - q);
 }
 
 // The three compare-and-swap steps of corner.py:607-629. With abs_sort the
@@ -376,17 +383,19 @@ __device__ __forceinline__ double frangi_gamma_sq(double gamma_sq_fixed,
 }
 
 // The vesselness of one voxel from its eigenvalues (ascending by magnitude)
-// and r_g: cuCIM's 2-D and 3-D inner kernels, statement by statement.
+// and r_g: cuCIM's 2-D and 3-D inner kernels, statement by statement, but for
+// the divisions by the three constants, which are products with their
+// reciprocals (na = -1 / alpha^2 and so on).
 template <class F>
 __device__ __forceinline__ F frangi_value(F lambda1, F lambda2, F lambda3, int nd, F r_g,
-                                          double alpha_sq, double beta_sq, double gamma_sq) {
+                                          double na, double nb, double ng) {
   F result;
   if (nd == 2) {
     F r_b;
     r_b = abs(lambda1) / max(lambda2, static_cast<F>(1.0e-10));
     r_b *= r_b;
-    result = exp(-r_b / beta_sq);
-    result *= 1.0 - exp(-r_g / gamma_sq);
+    result = exp(r_b * nb);
+    result *= 1.0 - exp(r_g * ng);
   } else {
     F r_a, r_b;
     F lam2 = max(lambda2, static_cast<F>(1.0e-10));
@@ -394,9 +403,9 @@ __device__ __forceinline__ F frangi_value(F lambda1, F lambda2, F lambda3, int n
     r_a = lam2 / lam3;
     r_a *= r_a;
     r_b = (lambda1 * lambda1) / (lam2 * lam3);
-    result = 1.0 - exp(-r_a / alpha_sq);
-    result *= exp(-r_b / beta_sq);
-    result *= 1.0 - exp(-r_g / gamma_sq);
+    result = 1.0 - exp(r_a * na);
+    result *= exp(r_b * nb);
+    result *= 1.0 - exp(r_g * ng);
   }
   return result;
 }
@@ -412,13 +421,13 @@ __global__ void k_frangi_inner(const F* __restrict__ l0, const F* __restrict__ l
                                const F* __restrict__ l2, int nd, int64_t n, double alpha_sq,
                                double beta_sq, double gamma_sq_fixed,
                                const unsigned long long* maxbits, F* out, int first) {
-  const double gamma_sq = frangi_gamma_sq(gamma_sq_fixed, maxbits);
+  const double na = -1.0 / alpha_sq, nb = -1.0 / beta_sq;
+  const double ng = -1.0 / frangi_gamma_sq(gamma_sq_fixed, maxbits);
   const F* ev[3] = {l0, l1, l2};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const F r_g = frangi_rg<F>(ev, nd, i);
-    const F result = frangi_value<F>(l0[i], l1[i], nd == 3 ? l2[i] : F(0), nd, r_g, alpha_sq,
-                                     beta_sq, gamma_sq);
+    const F result = frangi_value<F>(l0[i], l1[i], nd == 3 ? l2[i] : F(0), nd, r_g, na, nb, ng);
     out[i] = first ? result : frangi_fold(out[i], result);
   }
 }
@@ -434,7 +443,8 @@ __global__ void k_frangi_fused(const F* __restrict__ h0, const F* __restrict__ h
                                int64_t n, double alpha_sq, double beta_sq,
                                double gamma_sq_fixed, const unsigned long long* maxbits, F* out,
                                int first) {
-  const double gamma_sq = frangi_gamma_sq(gamma_sq_fixed, maxbits);
+  const double na = -1.0 / alpha_sq, nb = -1.0 / beta_sq;
+  const double ng = -1.0 / frangi_gamma_sq(gamma_sq_fixed, maxbits);
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     F lam1, lam2, lam3 = F(0);
@@ -466,7 +476,7 @@ __global__ void k_frangi_fused(const F* __restrict__ h0, const F* __restrict__ h
     }
     F r_g = fma(lam1, lam1, mul_rn(lam2, lam2));
     if (nd == 3) r_g = fma(lam3, lam3, r_g);
-    const F result = frangi_value<F>(lam1, lam2, lam3, nd, r_g, alpha_sq, beta_sq, gamma_sq);
+    const F result = frangi_value<F>(lam1, lam2, lam3, nd, r_g, na, nb, ng);
     out[i] = first ? result : frangi_fold(out[i], result);
   }
 }
