@@ -115,6 +115,9 @@ _sigs = {
     "cimx_gradient_magnitude": (
         [_A, _A, _P(CimxPass), ctypes.c_int, ctypes.c_int, ctypes.c_void_p], ctypes.c_int,
     ),
+    "cimx_edge_magnitude": (
+        [_A, _A, _P(CimxPass), ctypes.c_int, ctypes.c_int, ctypes.c_void_p], ctypes.c_int,
+    ),
     "cimx_laplace": (
         [_A, _A, _P(CimxPass), ctypes.c_int, ctypes.c_int, ctypes.c_void_p], ctypes.c_int,
     ),

@@ -552,6 +552,10 @@ int cimx_gradient_magnitude(const CimxArray* in, const CimxArray* out, const Cim
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t n = numel(out);
   if (n == 0) return CIMX_OK;
+  if (in->dtype == DT_F32) {
+    const int rc = try_grad2d(in, out, passes, naxes, passes_per_axis, st);
+    if (rc != CIMX_FUSED_DECLINED) return rc;
+  }
   const size_t bytes = (size_t)n * dtype_size(out->dtype);
   void* tmp = nullptr;
   if (naxes > 1) {

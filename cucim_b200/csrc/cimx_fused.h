@@ -65,6 +65,10 @@ inline int skip_kind(const float* w, int K, bool skip) {
 int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npasses,
               int lib_flags, cudaStream_t stream);
 
+// the magnitude of a 2-D image's two 3-tap gradient chains (cimx_edges.cu)
+int try_grad2d(const CimxArray* in, const CimxArray* out, const CimxPass* passes, int naxes,
+               int passes_per_axis, cudaStream_t st);
+
 // elementwise copy with conversion (used when a filter has no passes)
 int launch_copy_cast(const void* in, int tin, void* out, int tout, int64_t n,
                      cudaStream_t stream);

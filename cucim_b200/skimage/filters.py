@@ -4,6 +4,7 @@ _shared/filters.py:21-166, filters/edges.py:148-330 and :494,
 filters/ridges.py:50-595)."""
 
 import ctypes
+import functools
 import math
 from collections.abc import Iterable
 
@@ -139,6 +140,24 @@ def unsharp_mask(image, radius=1.0, amount=1.0, preserve_range=False, *, channel
     return _arrays.wrap_like(image, _unsharp_mask_single_channel(fimg, radius, amount, vrange))
 
 
+@functools.lru_cache(maxsize=256)
+def _edge_plan(edge_weights, smooth_weights, axes, ndim, mode):
+    """The passes of a gradient magnitude in float32, chain after chain, as
+    the library takes them; their number of chains and passes per chain; and
+    what the passes point into."""
+    fdt = np.dtype(np.float32)
+    ew = (np.asarray(edge_weights, dtype=fdt) / fdt.type(math.sqrt(ndim))).astype(fdt)
+    sw = np.asarray(smooth_weights, dtype=fdt)
+    lists = []
+    for ed in axes:
+        ed_n = ed % ndim
+        chain = [(ed_n, ew, mode, 0, True)]
+        chain += [(sd, sw, mode, 0, True) for sd in range(ndim) if sd != ed_n]
+        lists.append(ndi._build_passes(fdt, fdt, ndim, chain, 0.0, None))
+    items = [p for pl in lists for p in pl.items]
+    return (_lib.CimxPass * len(items))(*items), len(axes), ndim, lists
+
+
 def _generic_edge_filter(image, *, smooth_weights, edge_weights=(1, 0, -1), axis=None,
                          mode="reflect", cval=0.0):
     """edges.py:148-241: the edge taps along each requested axis, the
@@ -156,6 +175,18 @@ def _generic_edge_filter(image, *, smooth_weights, edge_weights=(1, 0, -1), axis
         axes = list(axis)
     magnitude = len(axes) > 1
     dt = _arrays.np_dtype(x)
+    if magnitude and dt.kind == "u" and dt.itemsize <= 2 and isinstance(mode, str):
+        # conversion, chains and magnitude in one call
+        check_mode(mode)
+        arr, naxes, per_axis, _ = _edge_plan(tuple(edge_weights), tuple(smooth_weights),
+                                             tuple(axes), ndim, mode)
+        xc = x.contiguous()
+        out = torch.empty(xc.shape, dtype=torch.float32, device=xc.device)
+        rc = _lib.lib.cimx_edge_magnitude(ctypes.byref(_arrays.to_cimx(xc)),
+                                          ctypes.byref(_arrays.to_cimx(out)), arr, naxes,
+                                          per_axis, _arrays.stream_of(xc))
+        _lib.check(rc, "edge magnitude")
+        return _arrays.wrap_like(image, out)
     if dt.kind == "f":
         fdt = supported_float_type(dt)
         image = _u.astype(image, fdt)

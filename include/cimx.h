@@ -234,6 +234,14 @@ CIMX_API int cimx_gradient_magnitude(const CimxArray* in, const CimxArray* out,
                             const CimxPass* passes, int naxes, int passes_per_axis,
                             void* stream);
 
+/* The same of img_as_float(in) (util/dtype.py:489-512), the magnitude that the
+ * skimage edge filters take of an integer image (filters/edges.py:148-241):
+ * `out` has the image's float type. uint8 / uint16 images with 3-tap chains in
+ * two dimensions are one launch. */
+CIMX_API int cimx_edge_magnitude(const CimxArray* in, const CimxArray* out,
+                                 const CimxPass* passes, int naxes, int passes_per_axis,
+                                 void* stream);
+
 /* Laplacian as a sum of per-axis chains: out = chain_0(in), then
  * tmp = chain_a(in); out += tmp (in out's dtype) for a >= 1. `passes` holds
  * naxes chains of passes_per_axis passes each (axis a's chain at

@@ -102,3 +102,22 @@ def test_mask_known_answer(filters):
 def test_mask_shape_mismatch(filters):
     with pytest.raises(ValueError):
         filters.sobel(dev(np.zeros((8, 9), np.float32)), dev(np.ones((8, 8), bool)))
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.float32])
+@pytest.mark.parametrize("name", ["sobel", "scharr", "prewitt"])
+@pytest.mark.parametrize("shape", [(1, 1), (1, 40), (33, 1), (2, 2), (8, 32), (63, 33), (65, 97)])
+def test_magnitude_in_one_launch(cuda, name, dtype, shape):
+    """The 2-D magnitude kernel around its 8 rows, 32 columns and the axes
+    shorter than the taps, against the oracle's separate passes."""
+    from cucim_b200.skimage import filters
+
+    r = np.random.default_rng(sum(shape))
+    if dtype == np.float32:
+        x = r.standard_normal(shape).astype(dtype)
+        x[0, -1], x[-1, shape[1] // 2] = np.inf, np.nan
+    else:
+        x = r.integers(0, np.iinfo(dtype).max + 1, shape).astype(dtype)
+    for mode in ("reflect", "mirror", "nearest", "constant", "wrap"):
+        got = getattr(filters, name)(torch.as_tensor(x).cuda(), mode=mode).cpu().numpy()
+        np.testing.assert_array_equal(got, FILTERS[name](x, mode=mode))
