@@ -69,6 +69,10 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
 int try_grad2d(const CimxArray* in, const CimxArray* out, const CimxPass* passes, int naxes,
                int passes_per_axis, cudaStream_t st);
 
+// the last two axes of a float64 array in one launch (cimx_strip_f64.cu)
+int try_strip_f64(const PassDesc& dy, const PassDesc& dx, const void* in, void* out,
+                  cudaStream_t st);
+
 // elementwise copy with conversion (used when a filter has no passes)
 int launch_copy_cast(const void* in, int tin, void* out, int tout, int64_t n,
                      cudaStream_t stream);

@@ -158,3 +158,18 @@ def test_long_passes(ndi, K, shape):
     xd = torch.as_tensor(flat).cuda()[1:].view(shape)
     got = ndi.correlate1d(xd, w, axis=0).cpu().numpy()
     np.testing.assert_array_equal(got, R.correlate1d(flat[1:].reshape(shape), w, 0))
+
+
+@pytest.mark.parametrize("K", [1, 3, 9, 10, 17, 18, 25, 33, 41, 42, 49, 50])
+@pytest.mark.parametrize("shape", [(8, 32), (17, 33), (2, 31, 207), (70, 257), (9, 700)])
+def test_float64_tail_passes(ndi, K, shape):
+    """Both tail passes of a float64 array in one launch (cimx_strip_f64.cu),
+    around its groups of 8 rows, 32 and 256 columns and the tap bounds."""
+    x = np.random.default_rng(K).standard_normal(shape)
+    x[..., 2, 5], x[..., 6, 20] = np.inf, np.nan
+    y, nd = x[..., ::-1].copy(), x.ndim
+    w, v = _taps(K, "plain"), _taps(max(K - 1, 1), "signed")
+    for mode in MODES:
+        _run(ndi, x, [(nd - 2, w, mode, 0), (nd - 1, w, mode, 0)], "float64", cval=1.25)
+        _run(ndi, y, [(nd - 2, v, mode, (v.size - 1) // 2), (nd - 1, w, mode, -(K // 2))],
+             "float64", cval=np.inf)
