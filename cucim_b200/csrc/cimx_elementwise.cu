@@ -6,6 +6,8 @@
 // cuCIM kernel it replaces (cited per kernel), so the compiler's rounding and
 // contraction decisions are the same ones cuCIM's kernels get.
 #include <algorithm>
+#include <cstring>
+#include <vector>
 #include <cmath>
 #include <vector>
 
@@ -88,6 +90,14 @@ template <class T>
 int launch_combine_t(void* acc, const void* t, int64_t n, int sub, cudaStream_t st) {
   k_combine<T><<<grid_for(n), 256, 0, st>>>(static_cast<T*>(acc), static_cast<const T*>(t), n, sub);
   return cuda_fail(cudaGetLastError(), "combine launch");
+}
+
+// whether two passes are the same filter along the same axis
+bool same_pass(const CimxPass& a, const CimxPass& b) {
+  return a.axis == b.axis && a.ntaps == b.ntaps && a.origin == b.origin && a.mode == b.mode &&
+         a.flags == b.flags && !(a.flags & CIMX_F_COMPLEX_TAPS) && a.ntaps > 0 && a.taps && b.taps &&
+         std::memcmp(&a.cval, &b.cval, sizeof(a.cval)) == 0 &&
+         std::memcmp(a.taps, b.taps, sizeof(double) * a.ntaps) == 0;
 }
 
 int launch_combine(void* acc, const void* t, int dt, int64_t n, int sub, cudaStream_t st) {
@@ -675,17 +685,47 @@ int cimx_laplace(const CimxArray* in, const CimxArray* out, const CimxPass* pass
   const int64_t n = numel(out);
   if (n == 0) return CIMX_OK;
   const size_t bytes = (size_t)n * dtype_size(out->dtype);
-  void* tmp = nullptr;
-  if (naxes > 1) {
-    tmp = scratch_alloc(bytes, st);
-    if (!tmp) return fail(CIMX_E_NOMEM, "scratch allocation for laplace failed");
-  }
+  int rc = cimx_separable(in, out, passes, passes_per_axis, 0, stream);
+  if (rc != CIMX_OK || naxes == 1) return rc;
+  void* tmp = scratch_alloc(bytes, st);
+  if (!tmp) return fail(CIMX_E_NOMEM, "scratch allocation for laplace failed");
   CimxArray t = *out;
   t.data = tmp;
-  int rc = cimx_separable(in, out, passes, passes_per_axis, 0, stream);
-  for (int a = 1; a < naxes && rc == CIMX_OK; ++a) {
-    rc = cimx_separable(in, &t, passes + (size_t)a * passes_per_axis, passes_per_axis, 0, stream);
-    if (rc == CIMX_OK) rc = launch_combine(out->data, tmp, out->dtype, n, 0, st);
+  // Chains after the first: float32 results whose last launch is a strip launch
+  // are added as they are stored; chains that begin with the same pass along the
+  // first axis share it (in tmp). Each value is rounded as the separate launches
+  // round it. Else: the chain into tmp, then a launch that adds it.
+  const CimxPass* shared = nullptr;  // the pass whose result tmp holds
+  for (int c = 1; c < naxes && rc == CIMX_OK; ++c) {
+    const CimxPass* chain = passes + (size_t)c * passes_per_axis;
+    int done = CIMX_FUSED_DECLINED;
+    if (in->dtype == DT_F32 && out->dtype == DT_F32 && passes_per_axis >= 1 && !tuning_needed(0)) {
+      std::vector<std::vector<double>> taps(passes_per_axis);
+      std::vector<PassDesc> ds(passes_per_axis);
+      for (int i = 0; i < passes_per_axis && rc == CIMX_OK; ++i)
+        rc = make_pass(in, chain[i], taps[i], ds[i]);
+      if (rc != CIMX_OK) break;
+      bool real = true;
+      for (const PassDesc& d : ds) real = real && !d.ctaps;
+      const bool pays = shared || (c + 1 < naxes && same_pass(chain[0], chain[passes_per_axis]));
+      if (real && passes_per_axis >= 2 && pays) {
+        if (!shared || !same_pass(*shared, chain[0])) {
+          rc = cimx_separable(in, &t, chain, 1, 0, stream);
+          shared = chain;
+        }
+        if (rc == CIMX_OK)
+          done = try_fused(&t, out, ds.data() + 1, passes_per_axis - 1, 0, st, true);
+      } else if (real) {
+        done = try_fused(in, out, ds.data(), passes_per_axis, 0, st, true);
+      }
+    }
+    if (rc == CIMX_OK && done == CIMX_FUSED_DECLINED) {
+      shared = nullptr;
+      rc = cimx_separable(in, &t, chain, passes_per_axis, 0, stream);
+      if (rc == CIMX_OK) rc = launch_combine(out->data, tmp, out->dtype, n, 0, st);
+    } else if (rc == CIMX_OK) {
+      rc = done;
+    }
   }
   scratch_free(tmp, bytes, st);
   return rc;

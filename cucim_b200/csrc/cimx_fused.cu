@@ -162,10 +162,11 @@ int try_vol(const CimxArray* in, const CimxArray* out, const PassDesc* ds, int z
 }  // namespace
 
 int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npasses,
-              int lib_flags, cudaStream_t st) {
+              int lib_flags, cudaStream_t st, bool add) {
   const int nd = in->ndim;
   const int D = out->dtype;
   if (npasses < 1 || npasses > CIMX_MAX_NDIM || nd < 1) return CIMX_FUSED_DECLINED;
+  if (add && D != DT_F32) return CIMX_FUSED_DECLINED;
   if (npasses == 2 && nd >= 2 && ds[0].axis == nd - 2 && ds[1].axis == nd - 1 &&
       in->dtype == DT_F64 && D == DT_F64)
     return try_strip_f64(ds[0], ds[1], in->data, out->data, st);
@@ -176,7 +177,7 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
     prev_axis = ds[i].axis;
   }
 
-  if (nd >= 3 && npasses == 3 && ds[0].axis == nd - 3 && ds[1].axis == nd - 2 &&
+  if (!add && nd >= 3 && npasses == 3 && ds[0].axis == nd - 3 && ds[1].axis == nd - 2 &&
       ds[2].axis == nd - 1 && !(lib_flags & CIMX_L_NO_VOLUME)) {
     static const int kChunks[4] = {0, 32, 64, 128};
     const int rc = try_vol(in, out, ds, kChunks[(lib_flags >> CIMX_L_ZCHUNK_SHIFT) & 3], st);
@@ -225,6 +226,7 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
     return fast;
   };
   if (!plan(false)) return CIMX_FUSED_DECLINED;
+  if (add && steps[nl - 1].kind != kStrip) return CIMX_FUSED_DECLINED;
 
   // ping-pong schedule: the last launch writes `out`
   const size_t tbytes = (size_t)n * dtype_size(D);
@@ -277,6 +279,7 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
           a.py.w[0] = 1.f;
         }
         a.has_x = 1;
+        a.add = add && j == nl - 1;
         fill_slab_pass(a.px, ds[s.x], tr[s.x], pass_in);
         rc = launch_strip(a, tsrc, D, st);
       }

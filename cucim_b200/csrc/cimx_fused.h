@@ -29,6 +29,7 @@ struct SlabArgs {
   void* out;
   long long B, Y, X;
   int has_y, has_x;  // has_y 0: py is the identity (one tap of 1)
+  int add;             // float32 results are added to what `out` holds
   SlabPass py, px;
 };
 
@@ -61,9 +62,11 @@ inline int skip_kind(const float* w, int K, bool skip) {
 
 // Runs the whole pass list `ds` (already resolved against the input shape)
 // in fast launches when they cover it. Returns CIMX_OK, a negative error, or
-// CIMX_FUSED_DECLINED (nothing was launched).
+// CIMX_FUSED_DECLINED (nothing was launched). `add` (float32): out += the
+// result, rounded like a pass of its own; declined unless the last launch is a
+// strip launch.
 int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npasses,
-              int lib_flags, cudaStream_t stream);
+              int lib_flags, cudaStream_t stream, bool add = false);
 
 // the magnitude of a 2-D image's two 3-tap gradient chains (cimx_edges.cu)
 int try_grad2d(const CimxArray* in, const CimxArray* out, const CimxPass* passes, int naxes,

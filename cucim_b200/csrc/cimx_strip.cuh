@@ -237,6 +237,25 @@ __device__ __forceinline__ void store_row(D* p, const float (&v)[kP], int left, 
   }
 }
 
+// v = old + v, old the outputs that store_row() is about to replace
+__device__ __forceinline__ void add_row(float (&v)[kP], const float* p, int left, int vec) {
+  if (vec > 0) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (4 * h < left) {
+        const float4 q = reinterpret_cast<const float4*>(p)[h];
+        v[4 * h] = __fadd_rn(q.x, v[4 * h]);
+        v[4 * h + 1] = __fadd_rn(q.y, v[4 * h + 1]);
+        v[4 * h + 2] = __fadd_rn(q.z, v[4 * h + 2]);
+        v[4 * h + 3] = __fadd_rn(q.w, v[4 * h + 3]);
+      }
+  } else {
+#pragma unroll
+    for (int e = 0; e < kP; ++e)
+      if (e < left) v[e] = __fadd_rn(p[e], v[e]);
+  }
+}
+
 // ---------------------------------------------------------------- strip
 
 // KY = 1: no y pass (rows are staged as they are, the x pass alone).
@@ -261,6 +280,7 @@ struct StripArgs {
   double cval_y, cval_x;
   int cin_y, cin_x, dt_y, dt_x;
   int trunc;           // truncating narrowing casts (narrow())
+  int add;             // float32: out += the result instead of out = it
   SlotTaps<KY, f2> y;  // in the last slots
   SlotTaps<KX, f2> x;  // in the first slots
 };
@@ -392,6 +412,8 @@ __global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
           float v[kP];
 #pragma unroll
           for (int p = 0; p < kP; ++p) v[p] = h ? hi2(acc[p]) : lo2(acc[p]);
+          if constexpr (sizeof(D) == 4)
+            if (a.add) add_row(v, orow, a.X - xo, a.vec_out);
           store_row<D>(orow, v, a.X - xo, a.vec_out, a.trunc);
         }
       }
@@ -589,6 +611,7 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
   a.cin_x = s.px.cval_as_input;
   a.dt_y = s.py.dt;
   a.dt_x = s.px.dt;
+  a.add = s.add;
   put_taps(a.y, s.py.w, s.py.K, s.py.skip, true);
   put_taps(a.x, s.px.w, s.px.K, s.px.skip, false);
   double bound = type_bound<T>();
