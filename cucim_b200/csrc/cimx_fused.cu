@@ -228,21 +228,31 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
   if (!plan(false)) return CIMX_FUSED_DECLINED;
   if (add && steps[nl - 1].kind != kStrip) return CIMX_FUSED_DECLINED;
 
-  // ping-pong schedule: the last launch writes `out`
+  // ping-pong schedule: the last launch writes `out`. With `add`, `out` holds
+  // the sum so far, which no other launch may touch: a second scratch buffer
+  // takes its turns.
   const size_t tbytes = (size_t)n * dtype_size(D);
-  void* temp = nullptr;
+  void *temp = nullptr, *temp2 = nullptr;
   if (nl >= 2) {
     temp = scratch_alloc(tbytes, st);
     // without scratch memory, both tail passes in one launch whatever their taps
     if (!temp && (!plan(true) || nl >= 2))
       return fail(CIMX_E_NOMEM, "scratch allocation for the ping-pong buffer failed");
   }
+  if (add && nl >= 3) {
+    temp2 = scratch_alloc(tbytes, st);
+    if (!temp2) {
+      scratch_free(temp, tbytes, st);
+      return CIMX_FUSED_DECLINED;
+    }
+  }
   int rc = CIMX_OK;
   const void* src = in->data;
   int tsrc = in->dtype;
   for (int j = 0; j < nl && rc == CIMX_OK; ++j) {
     const Step& s = steps[j];
-    void* dst = ((nl - 1 - j) % 2 == 0) ? out->data : temp;
+    void* const other = add ? temp2 : out->data;  // the buffer that takes turns with temp
+    void* dst = j == nl - 1 ? out->data : (nl - 1 - j) % 2 ? temp : other;
     switch (s.kind) {
       case kColumns: rc = launch_columns(ds[s.y], tr[s.y], tsrc, src, D, dst, st); break;
       case kGeneric: {
@@ -287,6 +297,7 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
     src = dst;
     tsrc = D;
   }
+  scratch_free(temp2, tbytes, st);
   scratch_free(temp, tbytes, st);
   // every check that can decline ran before the first launch
   return rc == CIMX_FUSED_DECLINED ? fail(CIMX_E_INVALID, "fast kernel missing") : rc;

@@ -74,6 +74,66 @@ def test_gaussian_laplace(ndi, mode, sigma):
     np.testing.assert_array_equal(got, R.gaussian_laplace(x, sigma, mode=mode, cval=-1.0))
 
 
+@pytest.mark.parametrize("shape,sigma,mode", [
+    ((12, 34, 40), 2.0, ("reflect", "nearest", "mirror")),
+    ((12, 34, 40), 3.0, ("reflect", "nearest", "mirror")),
+    ((12, 34, 40), 4.0, ("mirror", "wrap", "reflect")),
+    ((12, 34, 40), 5.0, ("reflect", "constant", "mirror")),
+    ((12, 34, 40), (1.0, 5.0, 3.0), ("nearest", "mirror", "wrap")),
+    ((5, 8, 34, 40), 1.0, "reflect"),
+    ((5, 8, 34, 40), 3.0, "mirror"),
+    ((5, 8, 34, 40), 5.0, "reflect"),
+    ((5, 8, 34, 40), 3.0, ("reflect", "nearest", "mirror", "wrap")),
+    ((5, 8, 34, 40), 1.0, ("reflect", "nearest", "mirror", "wrap")),
+    ((3, 4, 5, 33, 36), 1.0, "reflect"),
+    ((3, 4, 5, 33, 36), 1.0, ("reflect", "wrap", "nearest", "mirror", "constant")),
+])
+def test_gaussian_laplace_chains_of_many_launches(ndi, shape, sigma, mode):
+    """Chains of three launches and more that are added to the sum as they are
+    stored: long or unequal tail passes, more axes, and modes that keep the
+    chains from sharing their first pass."""
+    x = _data(shape, np.float32)
+    got = host(ndi.gaussian_laplace(dev(x), sigma, mode=mode, cval=0.5))
+    np.testing.assert_array_equal(got, R.gaussian_laplace(x, sigma, mode=mode, cval=0.5))
+
+
+def test_gaussian_laplace_with_two_scratch_volumes(ndi):
+    """Such a chain takes a third scratch volume; where there are only two, it
+    runs apart from the sum and is added by a launch of its own."""
+    import ctypes
+
+    from cucim_b200 import _lib
+
+    live, most = {}, []
+    fn = ctypes.CFUNCTYPE(ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p, ctypes.c_void_p)
+    rel = ctypes.CFUNCTYPE(None, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p,
+                           ctypes.c_void_p)
+
+    def give(n, *_):
+        most.append(len(live) + 1)
+        if len(live) == 2:
+            return None
+        t = torch.empty(n, dtype=torch.uint8, device="cuda")
+        live[t.data_ptr()] = t
+        return t.data_ptr()
+
+    def take(p, *_):
+        torch.cuda.synchronize()
+        del live[p]
+
+    alloc, free = fn(give), rel(take)
+    x = _data((12, 34, 40), np.float32)
+    mode = ("reflect", "nearest", "mirror")
+    set_allocator = _lib.lib.cimx_set_allocator
+    set_allocator(ctypes.cast(alloc, ctypes.c_void_p), ctypes.cast(free, ctypes.c_void_p), None)
+    try:
+        got = host(ndi.gaussian_laplace(dev(x), 3.0, mode=mode))
+    finally:
+        set_allocator(None, None, None)
+    assert max(most) == 3 and not live
+    np.testing.assert_array_equal(got, R.gaussian_laplace(x, 3.0, mode=mode))
+
+
 def test_gaussian_laplace_axes_dtypes_kwargs(ndi):
     x = _data((10, 30, 36), np.uint16)
     xd = dev(x)
