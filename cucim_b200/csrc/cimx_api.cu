@@ -108,6 +108,16 @@ bool c_contiguous(const CimxArray* a) {
   return true;
 }
 
+bool overlaps(const CimxArray* a, const CimxArray* b) {
+  const char* a0 = static_cast<const char*>(a->data);
+  const char* b0 = static_cast<const char*>(b->data);
+  const char* a1 = a0 + numel(a) * element_size(a->dtype);
+  const char* b1 = b0 + numel(b) * element_size(b->dtype);
+  return numel(a) > 0 && numel(b) > 0 && a0 < b1 && b0 < a1;
+}
+
+}  // namespace
+
 int check_array(const CimxArray* a, const char* name) {
   if (!a) return fail(CIMX_E_INVALID, std::string(name) + " is NULL");
   if (a->ndim < 0 || a->ndim > CIMX_MAX_NDIM)
@@ -128,16 +138,6 @@ int check_same_shape(const CimxArray* a, const CimxArray* b) {
     if (a->shape[d] != b->shape[d]) return fail(CIMX_E_INVALID, "output shape not correct");
   return CIMX_OK;
 }
-
-bool overlaps(const CimxArray* a, const CimxArray* b) {
-  const char* a0 = static_cast<const char*>(a->data);
-  const char* b0 = static_cast<const char*>(b->data);
-  const char* a1 = a0 + numel(a) * element_size(a->dtype);
-  const char* b1 = b0 + numel(b) * element_size(b->dtype);
-  return numel(a) > 0 && numel(b) > 0 && a0 < b1 && b0 < a1;
-}
-
-}  // namespace
 
 int check_mode(int mode) {
   if (mode < CIMX_MODE_REFLECT || mode > CIMX_MODE_CONSTANT)

@@ -146,7 +146,8 @@ __global__ void k_mask_erode_mul(F* __restrict__ res, const void* __restrict__ m
 
 // The magnitude of a 2-D image's two gradient chains in one launch: per axis an
 // edge pass along it and a smoothing pass along the other one, 3 centred taps
-// each, one boundary mode, fill value 0. `scale`: 1 / max of integer input.
+// each, one boundary mode, fill value 0. `out` has been checked (shape of `in`,
+// C-contiguous).
 int try_grad2d(const CimxArray* in, const CimxArray* out, const CimxPass* passes, int naxes,
                int passes_per_axis, cudaStream_t st) {
   if (in->ndim != 2 || naxes != 2 || passes_per_axis != 2 || out->dtype != DT_F32)
@@ -205,15 +206,16 @@ extern "C" int cimx_edge_magnitude(const CimxArray* in, const CimxArray* out,
     return cimx_gradient_magnitude(in, out, passes, naxes, passes_per_axis, stream);
   if (out->dtype != DT_F32 && out->dtype != DT_F64)
     return fail(CIMX_E_DTYPE, "edge magnitude output must be float32 or float64");
-  if (in->ndim != out->ndim) return fail(CIMX_E_INVALID, "output shape not correct");
+  int rc;
+  if ((rc = check_array(in, "input")) || (rc = check_array(out, "output")) ||
+      (rc = check_same_shape(in, out)))
+    return rc;
   int64_t n = 1;
-  for (int d = 0; d < in->ndim; ++d) {
-    if (in->shape[d] != out->shape[d]) return fail(CIMX_E_INVALID, "output shape not correct");
-    n *= in->shape[d];
-  }
+  for (int d = 0; d < in->ndim; ++d) n *= in->shape[d];
+  if (n == 0) return CIMX_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  int rc = try_grad2d(in, out, passes, naxes, passes_per_axis, st);
-  if (rc != CIMX_FUSED_DECLINED || n == 0) return n == 0 ? CIMX_OK : rc;
+  rc = try_grad2d(in, out, passes, naxes, passes_per_axis, st);
+  if (rc != CIMX_FUSED_DECLINED) return rc;
   // the image as floats, then the general path
   const size_t bytes = (size_t)n * dtype_size(out->dtype);
   CimxArray img = *out;

@@ -43,10 +43,13 @@ int fail(int code, const std::string& msg);
 int cuda_fail(cudaError_t e, const char* what);
 
 // Argument checks shared by every entry point that takes a CimxPass list
-// (cimx_api.cu): the boundary mode, and one pass resolved against the shape of
+// (cimx_api.cu): an array (extents, dtype, C-contiguous, data), two arrays of
+// one shape, the boundary mode, and one pass resolved against the shape of
 // `shape_of` into a PassDesc (taps copied into taps_store and flipped for
 // convolution, origin checked, anchor computed). in/out/dtypes are left for
 // the caller to fill.
+int check_array(const CimxArray* a, const char* name);
+int check_same_shape(const CimxArray* a, const CimxArray* b);
 int check_mode(int mode);
 int make_pass(const CimxArray* shape_of, const CimxPass& p, std::vector<double>& taps_store,
               PassDesc& d);

@@ -77,6 +77,33 @@ def test_validation_happens_before_device_work():
     assert _corr(good_in, good_out, K=0) == _lib.E_INVALID
 
 
+def test_edge_magnitude_checks_both_arrays():
+    """The one-launch magnitude writes its output densely: a strided output (a
+    region of a larger image) is refused like everywhere else, before any
+    device work (the pointers here are fake)."""
+    t, p = _lib.taps_pointer(np.ones(3))
+    passes = (_lib.CimxPass * 4)()
+    for i, axis in enumerate((0, 1, 1, 0)):
+        passes[i].axis, passes[i].ntaps, passes[i].mode, passes[i].taps = axis, 3, 0, p
+
+    def edge(a_in, a_out):
+        return _lib.lib.cimx_edge_magnitude(ctypes.byref(a_in), ctypes.byref(a_out), passes, 2, 2,
+                                            None)
+
+    for dtype in (np.uint8, np.uint16):
+        img, es = _arr((4, 5), dtype), np.dtype(dtype).itemsize
+        out = _arr((4, 5), np.float32, 0x9000)
+        assert edge(img, _arr((4, 5), np.float32, 0x9000, strides=(32, 4))) == _lib.E_LAYOUT
+        assert edge(img, _arr((4, 5), np.float32, 0x9000, strides=(4, 16))) == _lib.E_LAYOUT
+        assert edge(_arr((4, 5), dtype, strides=(8 * es, es)), out) == _lib.E_LAYOUT
+        assert edge(img, _arr((4, 6), np.float32, 0x9000)) == _lib.E_INVALID
+        assert edge(img, _arr((4, 5, 1), np.float32, 0x9000)) == _lib.E_INVALID
+        assert edge(img, _arr((4, 5), np.float32, 0)) == _lib.E_INVALID
+        assert edge(_arr((4, 5), dtype, 0), out) == _lib.E_INVALID
+        assert edge(img, _arr((4, 5), np.uint8 if es == 2 else np.uint16)) == _lib.E_DTYPE
+        assert edge(_arr((0, 5), dtype), _arr((0, 5), np.float32)) == 0
+
+
 def test_check_maps_errors_like_cucim():
     with pytest.raises(MemoryError):
         _lib.check(_lib.E_NOMEM, "x")
