@@ -195,8 +195,10 @@ __global__ void k_eig22(const F* __restrict__ M00, const F* __restrict__ M01,
 // feature/corner.py:566-647 — symmetric 3x3 eigenvalues, float64 inside
 // (Deledalle et al. closed form with the max(.,0) guards). Arguments are the
 // matrix [[a d f] [d b e] [f e c]]. Bound: the float64 pipe (half the float32
-// rate). 256^3 float32: 220 us against 331 with three cosines of divided angles;
-// with the vesselness (k_frangi_fused) 355 against 479.
+// rate). For float32 results the three cosines are angle sums, whose error (1.6
+// instead of 1.4e-16 of the norm for lam2) the rounding to float32 hides: 256^3
+// 220 us against 331 with three cosines of divided angles; with the vesselness
+// (k_frangi_fused) 355 against 479. float64 results keep the three cosines.
 template <class F>
 __device__ __forceinline__ void eig33(double a, double b, double c, double d, double e, double f,
                                       F& lam1, F& lam2, F& lam3) {
@@ -219,16 +221,23 @@ __device__ __forceinline__ void eig33(double a, double b, double c, double d, do
     phi = atan(sqrt(arg) / x2);
     if (x2 < 0) phi += M_PI;
   }
-  // cos((phi -+ pi) / 3) = cos(phi / 3) / 2 +- sin(phi / 3) sqrt(3) / 2: one
-  // sine and cosine for the three cosines and their three divisions
-  double sn, cs;
-  sincos(phi * (1.0 / 3.0), &sn, &cs);
   const double x1_term = (2.0 / 3.0) * sqrt(x1);
-  const double abc = (a + b + c) * (1.0 / 3.0);
-  const double h = 0.5 * cs, q = 0.86602540378443864676 * sn;
-  lam1 = abc - x1_term * cs;
-  lam2 = abc + x1_term * (h + q);
-  lam3 = abc + x1_term * (h - q);
+  if constexpr (sizeof(F) == 8) {
+    const double abc = (a + b + c) / 3.0;
+    lam1 = abc - x1_term * cos(phi / 3.0);
+    lam2 = abc + x1_term * cos((phi - M_PI) / 3.0);
+    lam3 = abc + x1_term * cos((phi + M_PI) / 3.0);
+  } else {
+    // cos((phi -+ pi) / 3) = cos(phi / 3) / 2 +- sin(phi / 3) sqrt(3) / 2: one
+    // sine and cosine for the three cosines and their three divisions
+    double sn, cs;
+    sincos(phi * (1.0 / 3.0), &sn, &cs);
+    const double abc = (a + b + c) * (1.0 / 3.0);
+    const double h = 0.5 * cs, q = 0.86602540378443864676 * sn;
+    lam1 = abc - x1_term * cs;
+    lam2 = abc + x1_term * (h + q);
+    lam3 = abc + x1_term * (h - q);
+  }
 }
 
 // The three compare-and-swap steps of corner.py:607-629. With abs_sort the
