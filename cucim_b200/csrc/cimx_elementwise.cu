@@ -6,9 +6,9 @@
 // cuCIM kernel it replaces (cited per kernel), so the compiler's rounding and
 // contraction decisions are the same ones cuCIM's kernels get.
 #include <algorithm>
-#include <cstring>
-#include <vector>
+#include <cfloat>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include <type_traits>
@@ -401,20 +401,37 @@ __device__ __forceinline__ double frangi_gamma_sq(double gamma_sq_fixed,
   return (s_max == 0) ? 2.0 : max(2 * gamma * gamma, 1e-10);
 }
 
+// -r / sq for a constant sq: the constant that frangi_value() takes, and the
+// quotient. float32: a product with the reciprocal, whose error the rounding of
+// the result hides; where the reciprocal of a tiny sq overflows, the largest
+// double gives the quotient's exp() all the same (0 for r = 0, beyond 1e260 for
+// any other float32). float64: the division itself.
+template <class F>
+__device__ __forceinline__ double frangi_const(double sq) {
+  if constexpr (sizeof(F) == 8) return sq;
+  const double n = -1.0 / sq;
+  return isinf(n) && sq != 0.0 ? copysign(DBL_MAX, n) : n;
+}
+template <class F>
+__device__ __forceinline__ double frangi_quotient(F r, double k) {
+  if constexpr (sizeof(F) == 8) return -r / k;
+  return r * k;
+}
+
 // The vesselness of one voxel from its eigenvalues (ascending by magnitude)
-// and r_g: cuCIM's 2-D and 3-D inner kernels, statement by statement, but for
-// the divisions by the three constants, which are products with their
-// reciprocals (na = -1 / alpha^2 and so on).
+// and r_g: cuCIM's 2-D and 3-D inner kernels, statement by statement, with the
+// quotients by alpha^2, beta^2 and gamma^2 (ka = frangi_const(alpha^2) and so
+// on) as frangi_quotient() forms them.
 template <class F>
 __device__ __forceinline__ F frangi_value(F lambda1, F lambda2, F lambda3, int nd, F r_g,
-                                          double na, double nb, double ng) {
+                                          double ka, double kb, double kg) {
   F result;
   if (nd == 2) {
     F r_b;
     r_b = abs(lambda1) / max(lambda2, static_cast<F>(1.0e-10));
     r_b *= r_b;
-    result = exp(r_b * nb);
-    result *= 1.0 - exp(r_g * ng);
+    result = exp(frangi_quotient(r_b, kb));
+    result *= 1.0 - exp(frangi_quotient(r_g, kg));
   } else {
     F r_a, r_b;
     F lam2 = max(lambda2, static_cast<F>(1.0e-10));
@@ -422,9 +439,9 @@ __device__ __forceinline__ F frangi_value(F lambda1, F lambda2, F lambda3, int n
     r_a = lam2 / lam3;
     r_a *= r_a;
     r_b = (lambda1 * lambda1) / (lam2 * lam3);
-    result = 1.0 - exp(r_a * na);
-    result *= exp(r_b * nb);
-    result *= 1.0 - exp(r_g * ng);
+    result = 1.0 - exp(frangi_quotient(r_a, ka));
+    result *= exp(frangi_quotient(r_b, kb));
+    result *= 1.0 - exp(frangi_quotient(r_g, kg));
   }
   return result;
 }
@@ -440,13 +457,13 @@ __global__ void k_frangi_inner(const F* __restrict__ l0, const F* __restrict__ l
                                const F* __restrict__ l2, int nd, int64_t n, double alpha_sq,
                                double beta_sq, double gamma_sq_fixed,
                                const unsigned long long* maxbits, F* out, int first) {
-  const double na = -1.0 / alpha_sq, nb = -1.0 / beta_sq;
-  const double ng = -1.0 / frangi_gamma_sq(gamma_sq_fixed, maxbits);
+  const double ka = frangi_const<F>(alpha_sq), kb = frangi_const<F>(beta_sq);
+  const double kg = frangi_const<F>(frangi_gamma_sq(gamma_sq_fixed, maxbits));
   const F* ev[3] = {l0, l1, l2};
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     const F r_g = frangi_rg<F>(ev, nd, i);
-    const F result = frangi_value<F>(l0[i], l1[i], nd == 3 ? l2[i] : F(0), nd, r_g, na, nb, ng);
+    const F result = frangi_value<F>(l0[i], l1[i], nd == 3 ? l2[i] : F(0), nd, r_g, ka, kb, kg);
     out[i] = first ? result : frangi_fold(out[i], result);
   }
 }
@@ -462,8 +479,8 @@ __global__ void k_frangi_fused(const F* __restrict__ h0, const F* __restrict__ h
                                int64_t n, double alpha_sq, double beta_sq,
                                double gamma_sq_fixed, const unsigned long long* maxbits, F* out,
                                int first) {
-  const double na = -1.0 / alpha_sq, nb = -1.0 / beta_sq;
-  const double ng = -1.0 / frangi_gamma_sq(gamma_sq_fixed, maxbits);
+  const double ka = frangi_const<F>(alpha_sq), kb = frangi_const<F>(beta_sq);
+  const double kg = frangi_const<F>(frangi_gamma_sq(gamma_sq_fixed, maxbits));
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
     F lam1, lam2, lam3 = F(0);
@@ -495,7 +512,7 @@ __global__ void k_frangi_fused(const F* __restrict__ h0, const F* __restrict__ h
     }
     F r_g = fma(lam1, lam1, mul_rn(lam2, lam2));
     if (nd == 3) r_g = fma(lam3, lam3, r_g);
-    const F result = frangi_value<F>(lam1, lam2, lam3, nd, r_g, na, nb, ng);
+    const F result = frangi_value<F>(lam1, lam2, lam3, nd, r_g, ka, kb, kg);
     out[i] = first ? result : frangi_fold(out[i], result);
   }
 }

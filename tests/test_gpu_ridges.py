@@ -95,6 +95,50 @@ def test_ridge_filters_float64(filters):
     frangi_close(host(filters.frangi(dev(x), sigmas=[1, 2])), R.frangi(x, sigmas=[1, 2]))
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("kw", [{"gamma": 1e-155}, {"alpha": 1e-155}, {"beta": 1e-155},
+                                {"gamma": 0.0}, {"alpha": 1e160, "gamma": 1e160}])
+def test_frangi_extreme_parameters(filters, dtype, kw):
+    """Squares of the parameters whose reciprocals overflow, zero and infinite
+    ones: flat regions (r_g = 0) stay 0 and not nan, like the quotients."""
+    x = np.zeros((24, 26), dtype)
+    x[10:12, 3:20] = 1
+    with np.errstate(all="ignore"):
+        exp = R.frangi(x, sigmas=[1, 2], black_ridges=False, **kw)
+    got = host(filters.frangi(dev(x), sigmas=[1, 2], black_ridges=False, **kw))
+    np.testing.assert_array_equal(np.isnan(got), np.isnan(exp))
+    np.testing.assert_allclose(got, exp, rtol=1e-6 if dtype == np.float32 else 1e-12, atol=1e-30)
+
+
+def test_float64_vesselness_keeps_its_precision(cuda):
+    """The vesselness of float64 eigenvalues whose squares are exact, with an
+    exponent near 10 that makes the quotient's rounding visible: no further from
+    the extended-precision value than the same statements in float64 on the host."""
+    import ctypes
+
+    from cucim_b200 import _arrays, _lib
+
+    n = 400_000
+    l1, l2 = np.random.default_rng(9).integers(900_000, 1_100_000, n) / 2.0 ** 20, np.ones(n)
+    beta, gamma = 0.24, 0.01  # gamma: the second factor is 1
+
+    def value(F):
+        return np.exp(-(l1.astype(F) ** 2) / F(2 * beta * beta))
+
+    ls = [dev(l1), dev(l2)]
+    out = torch.empty(n, dtype=torch.float64, device="cuda")
+    elems = (_lib.CimxArray * 2)(*[_arrays.to_cimx(t) for t in ls])
+    rc = _lib.lib.cimx_frangi_accumulate(elems, 2, ctypes.byref(_arrays.to_cimx(out)), 0.5,
+                                         beta, gamma, 1, None, _arrays.stream_of(out))
+    assert rc == 0, _lib.last_error()
+    exact = value(np.longdouble)
+
+    def rms(x):
+        return float(np.sqrt(np.mean(np.square((x - exact) / exact))))
+
+    assert rms(host(out)) <= 1.1 * rms(value(np.float64))
+
+
 def test_float64_eigenvalues_keep_their_precision(cuda):
     """Eigenvalues of 3 x 3 float64 matrices v v' + w w' (well conditioned in the
     largest one): no further from the extended-precision value of the closed form
