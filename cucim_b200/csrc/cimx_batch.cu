@@ -1,4 +1,4 @@
-// cimx_batch.cu — many uneven tiles in one persistent launch: for every
+// cimx_batch.cu — many uneven tiles in one launch: for every
 // uint8 RGB tile, rgb2gray, then a gaussian (its own sigma, mode 'nearest'),
 // then the sobel gradient magnitude (mode 'reflect'), float32 out — the
 // pipeline of skimage.color.rgb2gray -> skimage.filters.gaussian ->
@@ -14,9 +14,9 @@
 //           'reflect' borders, float32 intermediates;
 //   out   = sqrt(d0*d0 + d1*d1), each product and the sum rounded to float32.
 //
-// Work: a tile is cut into strips of up to 254 - 2r output columns and chunks
-// of up to 254 rows; a CTA walks down a strip, 16 rows at a time, on 256
-// staged columns:
+// Work: a tile is cut into strips of up to C - 2 - 2r output columns and chunks
+// of rows; a CTA of C threads walks down a strip, 16 rows at a time, on C staged
+// columns:
 //   * gray rows live in a ring in shared memory, the K - 1 + 16 rows that a
 //     group's y chains read: every pixel is converted once per strip (1.1 to
 //     1.35 times in all, for the halo columns) and its words are loaded while
@@ -27,19 +27,31 @@
 //   * x chains: a thread takes a row pair and 8 columns of the result;
 //   * edges and magnitude: a thread takes one column and 4 rows, so that a
 //     warp's stores cover consecutive floats at any alignment.
-// Two barriers per 16 rows, two CTAs per SM up to 65 taps (113 KB each, set by
-// the batch's largest radius).
+// Two barriers per 16 rows. C = 256: two CTAs per SM up to 65 taps (113 KB each,
+// set by the batch's largest radius). C = 128 up to 17 taps, where the halo of
+// narrow strips is short: four CTAs per SM, whose barriers and loads overlap, and
+// 64 x 64 tiles leave half as many columns idle (4000 of them, 5 / 17 taps, 225 /
+// 253 us against 362 / 407 with C = 256; 1000 of 128 x 128 227 / 247 against 205 /
+// 228; the mean over 1 to 4000 tiles of 32 to 4096 a side 0.87).
+//
+// Chunks have 14 to 510 rows (batch_groups): few tiles are cut into short ones,
+// or they would leave the chip idle (one tile of 1024^2 is 10 strips of 510 rows),
+// many tiles into long ones, which convert fewer halo rows. The tile table gives
+// every tile a range of block indexes; its items are spread evenly over that
+// range (find_item), so that consecutive CTAs take about one item each whatever
+// the tile sizes. 16 tiles of 256^2, 17 taps: 21 us, against 574 with 510-row
+// chunks whose indexes lay at the start of each range, a CTA's a grid apart.
 //
 // Bound: instruction issue, shared between the FMAs (about K (1 + 256 /
 // (254 - 2r)) per pixel) and the conversion and edge arithmetic (about 100
 // instructions per pixel), at 16 warps per SM with barriers (51 % of the issue
-// slots used). 1024 tiles of 64-1024 a side, sigmas 0.5-8: 3.15 ms; 64 x 64
-// blocks with a halo on all sides, whose gray region is 2.3 times the output
-// at 33 taps and 4.1 at 65, 6.99; chunks of 254 instead of 510 rows and
-// single-row edges 3.52.
+// slots used). 1024 tiles of 64-1024 a side, sigmas 0.5-8: 2.97 ms (3.16 with
+// the indexes a grid apart); 64 x 64 blocks with a halo on all sides, whose gray
+// region is 2.3 times the output at 33 taps and 4.1 at 65, 6.99.
 // The launch reads only device memory that the caller prepared, so it can
 // be captured in a CUDA graph and replayed.
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 
 #include "cimx_common.cuh"
@@ -50,12 +62,12 @@ namespace cimx {
 namespace {
 
 constexpr int kBT = 64;          // side of the blocks that the tile table counts
-constexpr int kBThreads = 256;
-constexpr int kBCols = 256;      // staged columns of a strip
+constexpr int kBCols = 256;      // staged columns of a strip and threads of its CTA
+constexpr int kBNarrow = 128;    // the same for short filters
 constexpr int kBG = 16;          // rows per group
-constexpr int kBRows = 32 * kBG - 2;  // output rows per chunk: 32 groups with the edge passes' halo
 constexpr int kBSRows = kBG + 2;      // smoothed rows kept for the edge passes
 constexpr int kBMaxTaps = 129;   // radius <= 64
+constexpr int kBNarrowTaps = 17;
 static_assert(sizeof(CimxBatchTile) == 56, "CimxBatchTile layout is part of the ABI");
 
 struct BatchArgs {
@@ -64,6 +76,9 @@ struct BatchArgs {
   long long nblocks;
   const float* taps;
   int max_r;
+  int rows;  // most output rows per chunk
+  int places;  // per block index
+  int per;   // places per CTA, at most one per warp
   float edge[3], smooth[3];
 };
 
@@ -103,20 +118,21 @@ using fast::pack2;
 // The x chains read up to 16 columns past a row pair: values that no stored
 // output uses, the last of them in S.
 constexpr int kTapBytes = (kBMaxTaps + 1) * 8;
-constexpr int kTPitch = kBCols * 8 + 16;
-constexpr int kTBytes = kBG / 2 * kTPitch;
+__host__ __device__ constexpr int t_pitch(int C) { return C * 8 + 16; }
+__host__ __device__ constexpr int t_bytes(int C) { return kBG / 2 * t_pitch(C); }
 __host__ __device__ constexpr int ring_rows(int K) { return (K - 1 + 7) / 8 * 8 + kBG; }
-__host__ __device__ constexpr int s_pitch(int K) { return (kBCols - (K - 1) + 7) / 8 * 8 + 4; }
+__host__ __device__ constexpr int s_pitch(int C, int K) { return (C - (K - 1) + 7) / 8 * 8 + 4; }
 // for K taps and fewer: S is widest for the shortest filter with K's ring, and
 // the next longer ring adds 8 KB against 8 columns of S
-__host__ __device__ constexpr int batch_smem(int K) {
-  const int widest = kBCols + 8 - (K - 1 + 7) / 8 * 8 + 4;
-  return kTapBytes + ring_rows(K) * kBCols * 4 + kTBytes + kBSRows * widest * 4;
+__host__ __device__ constexpr int batch_smem(int C, int K) {
+  const int widest = C + 8 - (K - 1 + 7) / 8 * 8 + 4;
+  return kTapBytes + ring_rows(K) * C * 4 + t_bytes(C) + kBSRows * widest * 4;
 }
-static_assert(batch_smem(65) <= 113 * 1024 - 256, "two CTAs per SM up to 65 taps");
-static_assert(batch_smem(kBMaxTaps) <= 223 * 1024, "longest filter");
-static_assert(kBCols - (kBMaxTaps - 1) - 2 >= kBT && kBRows >= kBT,
-              "a tile has no more strips and chunks than blocks");
+static_assert(batch_smem(kBCols, 65) <= 113 * 1024 - 256, "two CTAs per SM up to 65 taps");
+static_assert(batch_smem(kBCols, kBMaxTaps) <= 223 * 1024, "longest filter");
+static_assert(batch_smem(kBNarrow, kBNarrowTaps) <= 48 * 1024, "four CTAs per SM, no opt-in");
+static_assert(kBCols - (kBMaxTaps - 1) - 2 >= kBT && kBNarrow - (kBNarrowTaps - 1) - 2 >= kBT,
+              "a tile has no more strips than columns of blocks");
 
 // acc[p] = the chain over taps k = 0 .. K-1 of x(p + k) * w[k] for 8
 // consecutive outputs of two lines, taps ascending from +0. `load8(b, v)` gives
@@ -170,9 +186,11 @@ struct BatchItem {
   int tile, x0, xw, y0, rows;  // tile < 0: nothing to do
 };
 
-// The item of block index g. A tile's items take the first of its block
-// indexes, the others have none.
-__device__ __forceinline__ BatchItem find_item(const BatchArgs& a, long long g, int lane) {
+// The item of a place. Every block index has a.places of them; a tile's items are
+// spread over its places, the others have none.
+template <int C>
+__device__ __forceinline__ BatchItem find_item(const BatchArgs& a, long long place, int lane) {
+  const long long g = place / a.places;
   // the last tile whose first block <= g, found by a warp: each round probes 32
   // evenly spaced tiles of (lo, hi] and keeps the span between the last probe
   // <= g and the next one (three rounds for 4096 tiles)
@@ -192,17 +210,24 @@ __device__ __forceinline__ BatchItem find_item(const BatchArgs& a, long long g, 
   BatchItem it{-1, 0, 0, 0, 0};
   const CimxBatchTile& t = a.tiles[lo];
   const int K = t.ntaps, H = t.height, W = t.width;
-  const long long j = g - t.first_block;
+  const long long j = place - t.first_block * a.places;
   // a block index outside the tile (inconsistent table) is skipped
   if (j < 0 || K < 1 || K / 2 > a.max_r || H < 1 || W < 1) return it;
   const int r = K / 2;
-  const int wmax = kBCols - 2 - 2 * r;
-  const int nx = (W + wmax - 1) / wmax, ny = (H + kBRows - 1) / kBRows;
-  if (j >= static_cast<long long>(nx) * ny) return it;
+  const int wmax = C - 2 - 2 * r;
+  const long long np = (W + kBT - 1LL) / kBT * ((H + kBT - 1LL) / kBT) * a.places;
+  if (j >= np) return it;
+  const int nx = (W + wmax - 1) / wmax;
+  int ny = static_cast<int>(min((H + a.rows - 1LL) / a.rows, np / nx));
   const int xw = (W + nx - 1) / nx;
   const int rows = ((H + ny - 1) / ny + 2 + kBG - 1) / kBG * kBG - 2;
-  it.x0 = static_cast<int>(j % nx) * xw;
-  it.y0 = static_cast<int>(j / nx) * rows;
+  ny = (H + rows - 1) / rows;
+  // item k has place k np / (nx ny)
+  const long long ni = static_cast<long long>(nx) * ny;
+  const long long k = (j * ni + np - 1) / np;
+  if (k >= ni || k * np / ni != j) return it;
+  it.x0 = static_cast<int>(k % nx) * xw;
+  it.y0 = static_cast<int>(k / nx) * rows;
   it.xw = min(xw, W - it.x0);
   it.rows = min(rows, H - it.y0);
   if (it.xw > 0 && it.rows > 0) it.tile = lo;
@@ -210,24 +235,23 @@ __device__ __forceinline__ BatchItem find_item(const BatchArgs& a, long long g, 
 }
 
 // MID: the edge taps have a middle one
-template <bool MID>
-__global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const BatchArgs a) {
+template <int C, bool MID>
+__global__ void __launch_bounds__(C, 512 / C) k_batch_gray_gauss_sobel(const BatchArgs a) {
   extern __shared__ __align__(16) unsigned char sm_batch[];
-  __shared__ BatchItem s_item[kBThreads / 32];
+  __shared__ BatchItem s_item[C / 32];
+  constexpr int kTPitch = t_pitch(C);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  {
-    // one block index per warp, the CTA's indexes a grid apart: those of one
-    // tile's items, which lie together, go to different CTAs
-    const long long g = blockIdx.x + static_cast<long long>(warp) * gridDim.x;
+  if (warp < a.per) {  // one place per warp
+    const long long place = static_cast<long long>(blockIdx.x) * a.per + warp;
     BatchItem it{-1, 0, 0, 0, 0};
-    if (g < a.nblocks) it = find_item(a, g, lane);
+    if (place < a.nblocks * a.places) it = find_item<C>(a, place, lane);
     if (lane == 0) s_item[warp] = it;
   }
   __syncthreads();
   f2* const taps = reinterpret_cast<f2*>(sm_batch);
   float* const ring = reinterpret_cast<float*>(sm_batch + kTapBytes);
 
-  for (int n = 0; n < kBThreads / 32; ++n) {
+  for (int n = 0; n < a.per; ++n) {
     const BatchItem it = s_item[n];
     if (it.tile < 0) continue;  // the same for every thread
     const CimxBatchTile& t = a.tiles[it.tile];
@@ -237,9 +261,9 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
     const long long out_pitch = t.out_pitch > 0 ? t.out_pitch : W;
     const uint8_t* const rgb = t.rgb;
     float* const out = t.out;
-    const int R = ring_rows(K), SP = s_pitch(K);
-    unsigned char* const T = reinterpret_cast<unsigned char*>(ring + R * kBCols);
-    f2* const S = reinterpret_cast<f2*>(T + kTBytes);
+    const int R = ring_rows(K), SP = s_pitch(C, K);
+    unsigned char* const T = reinterpret_cast<unsigned char*>(ring + R * C);
+    f2* const S = reinterpret_cast<f2*>(T + t_bytes(C));
     // the smoothed row s of the walk is row ys + s of the tile, and the
     // smoothed column c is column x0 - 1 + c; gray row j is row ys - r + j,
     // gray column c is column x0 - 1 - r + c (both 'nearest')
@@ -248,7 +272,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
     const int need = ns + 2 * r;        // staged columns in use
     const int groups = (it.rows + 2 + kBG - 1) / kBG;
 
-    for (int k = tid; k < K; k += kBThreads) {
+    for (int k = tid; k < K; k += C) {
       const float w = a.taps[t.taps_offset + k];
       taps[k] = pack2(w, w);
     }
@@ -257,7 +281,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
     // their 12 bytes come from three or four aligned words (each holds at least
     // one of the bytes, so it lies in the tile's allocation); at its ends byte
     // by byte.
-    const int gc = (tid & 63) * 4, grow = tid >> 6;
+    const int gc = tid % (C / 4) * 4, grow = tid / (C / 4);
     const int xs = it.x0 - 1 - r + gc;
     const bool gon = gc < need;
     const bool words = xs >= 0 && xs + 3 < W;
@@ -300,7 +324,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
         const uint32_t v2 = __funnelshift_r(wv[u][2], wv[u][3], shv[u]);
         int q = slot + grow + 4 * u;
         if (q >= R) q -= R;
-        *reinterpret_cast<float4*>(ring + q * kBCols + gc) = make_float4(
+        *reinterpret_cast<float4*>(ring + q * C + gc) = make_float4(
             luma(v0 & 255u, (v0 >> 8) & 255u, (v0 >> 16) & 255u),
             luma(v0 >> 24, v1 & 255u, (v1 >> 8) & 255u),
             luma((v1 >> 16) & 255u, v1 >> 24, v2 & 255u),
@@ -328,16 +352,16 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
       if (more) gray_load(R + g * kBG);
       {
         // y chains: column pair p, rows 8 q .. 8 q + 7 of the group
-        const int p = tid & 127, q = tid >> 7;
+        const int p = tid % (C / 2), q = tid / (C / 2);
         if (2 * p < need) {
           int slot = base + 8 * q;
           if (slot >= R) slot -= R;
           const float* col = ring + 2 * p;
           f2 acc[8];
           chain8(acc, taps, K, [&](f2(&v)[8]) {
-            const float* at = col + slot * kBCols;
+            const float* at = col + slot * C;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const f2*>(at + j * kBCols);
+            for (int j = 0; j < 8; ++j) v[j] = *reinterpret_cast<const f2*>(at + j * C);
             slot += 8;
             if (slot == R) slot = 0;
           });
@@ -414,7 +438,7 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
                       fma2(v, pack2(a.smooth[1], a.smooth[1]),
                            fma2(u, pack2(a.smooth[0], a.smooth[0]), 0ull)));
         };
-        for (int c = (warp >> 2) * 32 + lane; c < it.xw; c += 64) {
+        for (int c = (warp >> 2) * 32 + lane; c < it.xw; c += C / 4) {
           f2 v[3][3], e1[3];
 #pragma unroll
           for (int i = 0; i < 3; ++i)
@@ -455,6 +479,32 @@ __global__ void __launch_bounds__(kBThreads, 2) k_batch_gray_gauss_sobel(const B
   }
 }
 
+// Row groups per chunk, from the batch's mean tile (its table is on the device):
+// whole waves of CTAs against the rows that every chunk converts and filters
+// again. The weights are microseconds of a lone CTA (one tile of 200 x 200, 5 to
+// 129 taps: 5 to 17 for an empty chunk, 4.2 to 7.5 a group); two on an SM take
+// 1.4 times as long.
+int batch_groups(long long nblocks, int ntiles, int C, int K) {
+  const double slots = 148.0 * (C == kBNarrow ? 4 : K <= 65 ? 2 : 1);
+  const int side = std::max(
+      kBT, static_cast<int>(kBT * std::sqrt(static_cast<double>(nblocks) / ntiles)));
+  const int nx = (side + C - 2 - K) / (C - 1 - K);
+  int groups = 0;
+  double best = 0;
+  for (int g : {1, 2, 3, 6, 16, 32}) {
+    const int ny = (side + kBG * g - 3) / (kBG * g - 2);
+    const int used = ((side + ny - 1) / ny + 2 + kBG - 1) / kBG;
+    const double item = 14 + 0.05 * K + used * (4.1 + 0.026 * K);
+    const double waves = static_cast<double>(ntiles) * nx * ny / slots;
+    const double cost = item * std::max(1.0, 0.8 * (waves + 0.8));
+    if (groups == 0 || cost < best) {
+      best = cost;
+      groups = g;
+    }
+  }
+  return groups;
+}
+
 }  // namespace
 }  // namespace cimx
 
@@ -480,24 +530,36 @@ extern "C" int cimx_batch_gray_gauss_sobel(const CimxBatchTile* tiles, int ntile
     a.edge[k] = edge_taps[k];
     a.smooth[k] = smooth_taps[k];
   }
-  const size_t smem = batch_smem(max_taps);
+  const bool narrow = max_taps <= kBNarrowTaps;
+  const int C = narrow ? kBNarrow : kBCols;
+  const size_t smem = batch_smem(C, max_taps);
   constexpr int kDynLimit = 223 * 1024;
-  auto* kern = edge_taps[1] != 0.f ? k_batch_gray_gauss_sobel<true> : k_batch_gray_gauss_sobel<false>;
+  using Kernel = void (*)(const BatchArgs);
+  static constexpr Kernel kKernels[2][2] = {
+      {k_batch_gray_gauss_sobel<kBCols, false>, k_batch_gray_gauss_sobel<kBCols, true>},
+      {k_batch_gray_gauss_sobel<kBNarrow, false>, k_batch_gray_gauss_sobel<kBNarrow, true>}};
+  const Kernel kern = kKernels[narrow][edge_taps[1] != 0.f];
   static std::once_flag once;
   static cudaError_t attr_err = cudaSuccess;
   std::call_once(once, [] {
-    for (auto* k : {k_batch_gray_gauss_sobel<true>, k_batch_gray_gauss_sobel<false>}) {
+    for (auto* k : kKernels[0]) {
       const cudaError_t e =
           cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kDynLimit);
       if (e != cudaSuccess) attr_err = e;
     }
   });
   if (attr_err != cudaSuccess) return cuda_fail(attr_err, "batch: shared memory attribute");
-  // a CTA takes one block index per warp; those without an item cost it the
-  // lookup alone
-  constexpr int kPer = kBThreads / 32;
-  const long long grid = (nblocks + kPer - 1) / kPer;
+  const int groups = batch_groups(nblocks, ntiles, C, max_taps);
+  a.rows = kBG * groups - 2;
+  a.places = std::max(1, 8 / groups);
+  // about one item per CTA; a place without one costs its lookup, of which few
+  // matter
+  const int wmax = C - 2 - 2 * a.max_r;
+  a.per = static_cast<int>(std::max(
+      1LL, std::min({nblocks * a.places / 1024, C / 32LL,
+                     (long long)wmax * a.rows / (kBT * kBT * a.places)})));
+  const long long grid = (nblocks * a.places + a.per - 1) / a.per;
   if (grid > 0x7fffffffLL) return fail(CIMX_E_INVALID, "batch: too many blocks");
-  kern<<<(unsigned)grid, kBThreads, smem, static_cast<cudaStream_t>(stream)>>>(a);
+  kern<<<(unsigned)grid, C, smem, static_cast<cudaStream_t>(stream)>>>(a);
   return cuda_fail(cudaGetLastError(), "batch launch");
 }

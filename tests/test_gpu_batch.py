@@ -147,12 +147,14 @@ def test_region_stream_rejects_bad_input(cuda):
         batch.RegionStream.from_regions(np.zeros((10, 10, 3), np.uint8), [(5, 5, 6, 2)], [1.0])
 
 
-# strips end at 254 - 2r output columns and chunks at 254 rows
+# strips end at 254 - 2r output columns (126 - 2r up to 17 taps); few tiles are
+# cut into chunks of 14 rows and more
 @pytest.mark.parametrize("sigma", [0.1, 0.5, 2.0, 3.7, 8.0, 16.0])
 def test_batch_strip_edges(cuda, sigma):
     from cucim_b200 import batch
 
-    wmax = 254 - 2 * int(4 * sigma + 0.5)
+    r = int(4 * sigma + 0.5)
+    wmax = (126 if r <= 8 else 254) - 2 * r
     shapes = [(14, wmax), (15, wmax + 1), (254, 9), (255, wmax - 1), (508, 2 * wmax + 1), (2, 1),
               (1, 7), (31, 2 * wmax)]
     tiles = _tiles(shapes, 8)
@@ -164,3 +166,24 @@ def test_batch_strip_edges(cuda, sigma):
     torch.cuda.synchronize()
     for g, r, t in zip(got, ref, tiles):
         assert torch.equal(g, r), (tuple(t.shape), (g - r).abs().max().item())
+
+
+@pytest.mark.parametrize("sigma", [0.5, 2.0, 2.2, 8.0])
+@pytest.mark.parametrize("count,shapes", [
+    (1, [(511, 300)]), (1, [(30, 1000)]), (1, [(1021, 64)]), (3, [(64, 64), (47, 63), (200, 129)]),
+    (40, [(95, 257), (64, 65)]), (300, [(64, 64)]), (300, [(130, 127), (46, 300), (16, 16)]),
+    (2500, [(64, 64), (63, 66)]), (400, [(509, 250), (510, 130), (511, 64), (1021, 190)]),
+])
+def test_batch_chunks_by_tile_count(cuda, count, shapes, sigma):
+    """The rows per chunk and the block indexes per CTA follow the batch's size:
+    from one tile in chunks of 14 rows to batches in chunks of 510 rows, each
+    tile's result the same."""
+    from cucim_b200 import batch
+
+    distinct = _tiles(shapes, 10)
+    ref = batch.gray_gauss_sobel_per_tile(distinct, [sigma] * len(distinct))
+    got = batch.TileBatch([distinct[i % len(distinct)] for i in range(count)],
+                          [sigma] * count).run()
+    assert len(got) == count
+    for i, g in enumerate(got):
+        assert torch.equal(g, ref[i % len(ref)]), (i, tuple(g.shape))
