@@ -264,6 +264,8 @@ __device__ __forceinline__ void add_row(float (&v)[kP], const float* p, int left
 // three CTAs: 96 bytes spilled, 128 x 1024^2 in 474 us against 238 at two).
 constexpr int kStripThreads = 256;
 constexpr int kLongThreads = 224;  // beyond kSlabMaxK taps: shared memory
+constexpr int kShortThreads = 128;
+constexpr int kShortTaps = 5;
 template <class T> constexpr int strip_ctas(int KY) { return KY <= (sizeof(T) == 4 ? 5 : 9) ? 3 : 2; }
 
 template <int KY, int KX>
@@ -281,12 +283,25 @@ struct StripArgs {
   int cin_y, cin_x, dt_y, dt_x;
   int trunc;           // truncating narrowing casts (narrow())
   int add;             // float32: out += the result instead of out = it
+  int group;           // SHORT: rows per group, whole slabs
+  short src[kG * kShortTaps];  // SHORT: row of the group that [row][y tap slot] reads, -1: fill
   SlotTaps<KY, f2> y;  // in the last slots
   SlotTaps<KX, f2> x;  // in the first slots
 };
 
-template <class T, class D, int KY, int KX, int NP, bool GEN>
-__global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
+//
+// SHORT: slabs of up to kG rows and up to kShortTaps taps. A group of kG rows
+// that ends with the slab would be mostly waste, so the rows of all slabs form
+// one (1, B Y, X) slab and a group takes whole slabs of it: each row is loaded
+// once, and as the row that a tap reads depends on the slab's rows and the mode
+// (a.src), a thread's column passes through shared memory of its own, which
+// other threads do not touch. 2^24 elements, 3 taps, slabs of 1 / 2 / 4 / 8 rows
+// of 1024, float32: 43 / 43 / 43 / 43 us against 294 / 154 / 84 / 49 with a group
+// per slab, uint8 43 / 43 / 43 / 43 against 332 / 173 / 92 / 53; rows of 64: 68 /
+// 68 / 67 / 66 against 437 / 249 / 147 / 82; 10 rows and more 58 / 57.
+template <class T, class D, int KY, int KX, int NP, bool GEN, bool SHORT>
+__global__ void __launch_bounds__(SHORT ? kShortThreads : kStripThreads,
+                                  SHORT ? 6 : strip_ctas<T>(KY))
     k_strip(const __grid_constant__ StripArgs<KY, KX> a) {
   extern __shared__ __align__(16) unsigned char sm_strip[];
   const int t = threadIdx.x, NT = blockDim.x;
@@ -315,6 +330,8 @@ __global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
   const unsigned char* win0 = sm_strip + (xwork ? rp : 0) * rs + cg * mid_off(kP);
   unsigned char* put0 = sm_strip + mid_off(2 * t);
   const int xo = x0 + cg * kP;
+  const int group = SHORT ? a.group : kG;
+  f2* const own = reinterpret_cast<f2*>(sm_strip + 2 * kRP * rs) + t;  // SHORT: [row * NT]
 
   for (long long b = blockIdx.y; b < a.B; b += gridDim.y) {
     const T* in = static_cast<const T*>(a.in) + b * a.Y * a.X + c0;
@@ -324,19 +341,20 @@ __global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
     // r0 + g0 - ay - (KY - ky) + i; slots below KY - ky are not read
     f2 win[KY + kG - 1];
     typename Raw<T>::type next[kG];
-    int r = r0 - a.ay - (KY - a.y.K);
+    int r = SHORT ? r0 - (KY - 1) : r0 - a.ay - (KY - a.y.K);
 #pragma unroll
-    for (int i = 0; i < KY - 1; i += kG) {
+    for (int i = 0; !SHORT && i < KY - 1; i += kG) {
       const uint32_t fill = load_rows<T>(next, in, d1, vec, r + i, a.Y, a.X, a.my);
 #pragma unroll
       for (int g = 0; g < kG && i + g < KY - 1; ++g)
         win[i + g] = (fill >> g) & 1u ? pack2(cy, cy) : widen<T>(next[g]);
     }
     r += KY - 1;  // row of next[0]
-    uint32_t fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, a.my);
+    const int my = SHORT ? CIMX_MODE_NEAREST : a.my;
+    uint32_t fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, my);
 
     int par = 0;
-    for (int g0 = 0; g0 < n; g0 += kG, par ^= 1) {
+    for (int g0 = 0; g0 < n; g0 += group, par ^= 1) {
 #pragma unroll
       for (int g = 0; g < kG; ++g) win[KY - 1 + g] = widen<T>(next[g]);
       if (fill) {
@@ -344,10 +362,26 @@ __global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
         for (int g = 0; g < kG; ++g)
           if ((fill >> g) & 1u) win[KY - 1 + g] = pack2(cy, cy);
       }
-      r += kG;
+      r += group;
+      if constexpr (SHORT) {
+#pragma unroll
+        for (int g = 0; g < kG; ++g) own[g * NT] = win[KY - 1 + g];
+      }
       {
         f2 acc[kG];
-        if constexpr (KY == 1) {
+        if constexpr (SHORT) {
+#pragma unroll
+          for (int g = 0; g < kG; ++g) acc[g] = 0ull;
+#pragma unroll
+          for (int k = 0; k < KY; ++k)
+            if (tap_on<KY, NP, GEN, true>(k, a.y.K, a.y.centre, a.y.act)) {
+#pragma unroll
+              for (int g = 0; g < kG; ++g) {
+                const int i = a.src[g * KY + k];
+                acc[g] = fma2(i < 0 ? pack2(cy, cy) : own[i * NT], a.y.w[k], acc[g]);
+              }
+            }
+        } else if constexpr (KY == 1) {
 #pragma unroll
           for (int g = 0; g < kG; ++g) acc[g] = win[g];
         } else {
@@ -378,8 +412,8 @@ __global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
               make_float4(lo2(acc[2 * q]), lo2(acc[2 * q + 1]), hi2(acc[2 * q]), hi2(acc[2 * q + 1]));
       }
 #pragma unroll
-      for (int i = 0; i < KY - 1; ++i) win[i] = win[i + kG];
-      if (g0 + kG < n) fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, a.my);
+      for (int i = 0; !SHORT && i < KY - 1; ++i) win[i] = win[i + kG];
+      if (g0 + group < n) fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, my);
       __syncthreads();
       if (xwarp) {
         const unsigned char* src = win0 + par * kRP * rs;
@@ -408,7 +442,7 @@ __global__ void __launch_bounds__(kStripThreads, strip_ctas<T>(KY))
         D* orow = out + static_cast<long long>(g0) * a.X + xo;
 #pragma unroll
         for (int h = 0; h < 2; ++h, orow += a.X) {
-          if (!(xwork && g0 + 2 * rp + h < n)) continue;
+          if (!(xwork && g0 + 2 * rp + h < n && (!SHORT || 2 * rp + h < group))) continue;
           float v[kP];
 #pragma unroll
           for (int p = 0; p < kP; ++p) v[p] = h ? hi2(acc[p]) : lo2(acc[p]);
@@ -565,7 +599,8 @@ inline int choose_chunk(long long rows, double cols, double slots, int G, double
     consider(c);
     if (c <= G) return static_cast<int>(chunk);
   }
-  for (long long c = rows / 64 / G * G; c >= G; c -= (c / 8 + G - 1) / G * G) consider(c);
+  for (long long c = rows / 64 / G * G; c >= G; c -= std::max<long long>(1, (c / 8 + G - 1) / G) * G)
+    consider(c);
   return static_cast<int>(chunk);
 }
 
@@ -593,8 +628,14 @@ static_assert(smem_bytes<kLongMaxK>(kLongThreads) <= 48 * 1024 &&
                   smem_bytes<kSlabMaxK>(kStripThreads) <= 48 * 1024,
               "no opt-in shared memory");
 
-template <class T, class D, int KY, int KX, int NP, bool GEN>
-int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
+template <class T, class D, int KY, int KX, int NP, bool GEN, bool SHORT = false>
+int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
+  static_assert(!SHORT || KY == kShortTaps, "table size");
+  SlabArgs s = slabs;
+  if (SHORT) {
+    s.Y *= s.B;
+    s.B = 1;
+  }
   StripArgs<KY, KX> a{};
   a.in = s.in;
   a.out = s.out;
@@ -622,14 +663,26 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
               : a.X % 4 == 0 && aligned(a.out, 4 * sizeof(D)) ? 1
                                                                 : 0;
 
-  auto* kern = k_strip<T, D, KY, KX, NP, GEN>;
+  a.group = kG;
+  if (SHORT) {
+    const int L = static_cast<int>(slabs.Y), lead = KY - s.py.K;
+    a.group = kG / L * L;
+    for (int g = 0; g < a.group; ++g)
+      for (int k = 0; k < s.py.K; ++k) {
+        const int m = map_coord32(g % L - s.py.anchor + k, L, s.py.mode);
+        a.src[g * KY + lead + k] = static_cast<short>(m < 0 ? -1 : g / L * L + m);
+      }
+  }
+  constexpr int kMost = SHORT ? kShortThreads : KX > kSlabMaxK ? kLongThreads : kStripThreads;
+  auto smem = [](int nt) { return smem_bytes<KX>(nt) + (SHORT ? kG * nt * (int)sizeof(f2) : 0); };
+
+  auto* kern = k_strip<T, D, KY, KX, NP, GEN, SHORT>;
   static int occ[kStripThreads / 32 + 1] = {};  // resident CTAs per SM, by warps
   static std::once_flag once;
   std::call_once(once, [&] {
-    for (int nt = 64; nt <= (KX > kSlabMaxK ? kLongThreads : kStripThreads); nt += 32) {
+    for (int nt = 64; nt <= kMost; nt += 32) {
       int v = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, nt, smem_bytes<KX>(nt)) != cudaSuccess ||
-          v < 1)
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, nt, smem(nt)) != cudaSuccess || v < 1)
         v = 1;
       occ[nt / 32] = v;
     }
@@ -637,14 +690,14 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
   // the last shape's geometry, so that repeated calls skip the search
   struct Shape {
     long long B, Y, X;
-    int ky, kx, nt, xw, tiles_x, chunk;
+    int ky, kx, group, nt, xw, tiles_x, chunk;
   };
   thread_local Shape last{};
-  if (last.B != s.B || last.Y != s.Y || last.X != s.X || last.ky != a.y.K || last.kx != a.x.K) {
+  if (last.B != s.B || last.Y != s.Y || last.X != s.X || last.ky != a.y.K || last.kx != a.x.K ||
+      last.group != a.group) {
     // CTA width: the staged columns of all tiles together as few as possible
     int nt = 0;
     long long tiles = 0, best = 0;
-    constexpr int kMost = KX > kSlabMaxK ? kLongThreads : kStripThreads;
     for (int w = 64; w <= kMost; w += 32) {
       int xw = (2 * w - (a.x.K - 1)) / 16 * 16;
       // long filters: four warps of x work, one per scheduler, of the six or
@@ -663,9 +716,9 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
     }
     const int xw = static_cast<int>(((s.X + tiles - 1) / tiles + 15) / 16 * 16);
     const int tiles_x = static_cast<int>((s.X + xw - 1) / xw);
-    const int chunk = choose_chunk(s.Y, (double)tiles_x * s.B, 148.0 * occ[nt / 32], kG,
+    const int chunk = choose_chunk(s.Y, (double)tiles_x * s.B, 148.0 * occ[nt / 32], a.group,
                                    a.y.K + a.x.K + 6, 4.0 * a.y.K + 150);
-    last = Shape{s.B, s.Y, s.X, a.y.K, a.x.K, nt, xw, tiles_x, chunk};
+    last = Shape{s.B, s.Y, s.X, a.y.K, a.x.K, a.group, nt, xw, tiles_x, chunk};
   }
   const int nt = last.nt;
   a.xw = last.xw;
@@ -674,7 +727,7 @@ int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
   const long long gx = ((s.Y + a.chunk - 1) / a.chunk) * a.tiles_x;
   if (gx > 0x7fffffffLL) return CIMX_FUSED_DECLINED;
   const dim3 grid((unsigned)gx, (unsigned)std::min<long long>(s.B, 65535));
-  kern<<<grid, nt, smem_bytes<KX>(nt), st>>>(a);
+  kern<<<grid, nt, smem(nt), st>>>(a);
   return cuda_fail(cudaGetLastError(), "strip launch");
 }
 
@@ -760,7 +813,11 @@ int launch_strip_td(const SlabArgs& s, cudaStream_t st) {
   }
   constexpr int kStep = kt_step(sizeof(T));
   switch (kt) {
-    case 5: return launch_strip_k<T, D, 5, 5, 5, false>(s, st);
+    case 5:
+      // from 9 rows on, a group would be a part of a slab
+      if (s.Y <= kG && s.B * s.Y < (1LL << 30))
+        return launch_strip_k<T, D, 5, 5, 5, false, true>(s, st);
+      return launch_strip_k<T, D, 5, 5, 5, false>(s, st);
     case 9: return launch_strip_k<T, D, 9, 9, 4, false>(s, st);
 #define CIMX_KT(K_) case K_: return launch_strip_k<T, D, K_, K_, kStep, false>(s, st);
     CIMX_KT(17) CIMX_KT(25) CIMX_KT(33)

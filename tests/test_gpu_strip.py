@@ -101,6 +101,29 @@ def test_tile_edges(ndi, rows, cols):
 
 
 @pytest.mark.parametrize("pair", PAIRS, ids=lambda p: "-".join(p))
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 5, 6, 7, 8])
+def test_short_slabs(ndi, pair, rows):
+    """Slabs of up to 8 rows with up to 5 taps share groups of rows: whole slabs
+    per group, slab counts around it, axes shorter than the taps."""
+    for count in (1, 2, 8 // rows, 8 // rows + 1, 37):
+        for cols in (3, 70, 253, 600):
+            x = _data((count, rows, cols), pair[0], count + cols)
+            if pair[0] == "float32":
+                x[0, 0, 1], x[-1, -1, 2] = np.inf, np.nan
+            for ky, kx, kind in ((3, 5, "plain"), (5, 3, "signed"), (4, 2, "plain"),
+                                 (3, 3, "centre"), (1, 5, "plain")):
+                wy, wx = _taps(ky, kind if ky > 1 else "plain"), _taps(kx, kind)
+                mode = MODES[(ky + kx + cols + count) % 5]
+                _run(ndi, x, [(1, wy, mode, 0), (2, wx, "reflect", 0)], pair[1], cval=2.0)
+                _run(ndi, x, [(1, wy, "constant", (ky - 1) // 2), (2, wx, mode, -(kx // 2))],
+                     pair[1], cval=7.0)
+    x = _data((4000, rows, 90), pair[0], rows)  # several groups per chunk
+    for mode in MODES:
+        _run(ndi, x, [(1, _taps(5, "plain"), mode, 0), (2, _taps(3, "plain"), mode, 0)], pair[1],
+             cval=1.0)
+
+
+@pytest.mark.parametrize("pair", PAIRS, ids=lambda p: "-".join(p))
 @pytest.mark.parametrize("offset", [0, 1, 2, 3])
 def test_base_alignment(ndi, pair, offset):
     """Contiguous arrays whose first element lies off the vector boundary."""
