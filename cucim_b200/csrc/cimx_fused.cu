@@ -216,6 +216,7 @@ int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npass
           s = {kStrip, i, i + 1};
           ++i;
         } else if (ds[i].inner >= kColumnsMinInner &&
+                   (tr[i].K <= kSlabMaxK || ring_long(ds[i].L, ds[i].inner, tr[i].K)) &&
                    (ds[i].axis == nd - 2 || !(lib_flags & CIMX_L_NO_STREAM))) {
           s.kind = kColumns;
         }

@@ -86,6 +86,15 @@ int launch_copy_cast(const void* in, int tin, void* out, int tout, int64_t n,
 // 124 / 42, 41 taps 126 / 39 against 160 / 50, 65 taps 181 / 56 against 213 / 73.
 // A step is 64 rows: shorter axes leave its warps idle.
 inline bool ring_takes(int64_t L, int K) { return K > kSlabMaxK || (K >= 22 && L >= 48); }
+// Whether a pass beyond kSlabMaxK taps takes it at all, or the generic kernel. Not
+// where half of its 64 columns are idle and a tile of the generic kernel is exactly
+// as wide (524 x 1000 x 32, 97 / 129 taps: 146 / 181 us against 123 / 148; 508 x
+// 1000 x 33 206 / 250 against 217 / 265), nor along two samples on unaligned rows,
+// whose folding every 4-byte copy repeats (167772 x 2 x 50, 66 / 97 / 129 taps:
+// 3.8 / 5.6 / 8.5 ms against 4.2 / 5.3 / 6.6).
+inline bool ring_long(int64_t L, int64_t inner, int K) {
+  return !(inner == 32 && L >= 64) && !(L == 2 && inner % 4 != 0 && K > 81);
+}
 int launch_ring_f32(const PassDesc& d, const float* w, int K, int anchor, bool skip,
                     const void* in, void* out, cudaStream_t st);
 

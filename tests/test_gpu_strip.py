@@ -164,7 +164,8 @@ def test_long_tail_passes_without_scratch_memory(ndi):
 
 
 @pytest.mark.parametrize("K", [22, 25, 26, 57, 66, 73, 74, 97, 128, 129, 130])
-@pytest.mark.parametrize("shape", [(150, 70), (64, 321), (41, 129), (257, 33), (300, 64)])
+@pytest.mark.parametrize("shape", [(150, 70), (64, 321), (41, 129), (257, 33), (300, 64),
+                                   (63, 32), (64, 32)])
 def test_long_passes(ndi, K, shape):
     """Long passes each in a launch of their own (cimx_ring.cuh along a strided
     axis), around its step of 64 rows, 64 columns and the tap bounds."""
