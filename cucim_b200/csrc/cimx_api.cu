@@ -309,7 +309,13 @@ int cimx_separable(const CimxArray* in, const CimxArray* out, const CimxPass* pa
   const size_t tbytes = (size_t)n * dtype_size(out->dtype);
   if (npasses > 1) {
     temp = scratch_alloc(tbytes, st);
-    if (!temp) return fail(CIMX_E_NOMEM, "scratch allocation for the ping-pong buffer failed");
+    if (!temp) {
+      rc = CIMX_FUSED_DECLINED;
+      if (!any_tensor && !(lib_flags & CIMX_L_NO_FUSION))
+        rc = try_fused(in, out, ds.data(), npasses, lib_flags, st, false, true);
+      if (rc != CIMX_FUSED_DECLINED) return rc;
+      return fail(CIMX_E_NOMEM, "scratch allocation for the ping-pong buffer failed");
+    }
   }
   const void* src = in->data;
   int tsrc = in->dtype;

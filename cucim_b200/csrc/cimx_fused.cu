@@ -162,14 +162,14 @@ int try_vol(const CimxArray* in, const CimxArray* out, const PassDesc* ds, int z
 }  // namespace
 
 int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npasses,
-              int lib_flags, cudaStream_t st, bool add) {
+              int lib_flags, cudaStream_t st, bool add, bool no_scratch) {
   const int nd = in->ndim;
   const int D = out->dtype;
   if (npasses < 1 || npasses > CIMX_MAX_NDIM || nd < 1) return CIMX_FUSED_DECLINED;
   if (add && D != DT_F32) return CIMX_FUSED_DECLINED;
   if (npasses == 2 && nd >= 2 && ds[0].axis == nd - 2 && ds[1].axis == nd - 1 &&
       in->dtype == DT_F64 && D == DT_F64)
-    return try_strip_f64(ds[0], ds[1], in->data, out->data, st);
+    return try_strip_f64(ds[0], ds[1], in->data, out->data, st, no_scratch);
   // passes in strictly ascending axis order, float32 weights
   int prev_axis = -1;
   for (int i = 0; i < npasses; ++i) {

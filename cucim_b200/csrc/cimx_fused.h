@@ -64,9 +64,10 @@ inline int skip_kind(const float* w, int K, bool skip) {
 // in fast launches when they cover it. Returns CIMX_OK, a negative error, or
 // CIMX_FUSED_DECLINED (nothing was launched). `add` (float32): out += the
 // result, rounded like a pass of its own; declined unless the last launch is a
-// strip launch.
+// strip launch. `no_scratch`: there is no scratch memory, so that kernels without
+// any are taken where others would be faster.
 int try_fused(const CimxArray* in, const CimxArray* out, PassDesc* ds, int npasses,
-              int lib_flags, cudaStream_t stream, bool add = false);
+              int lib_flags, cudaStream_t stream, bool add = false, bool no_scratch = false);
 
 // the magnitude of a 2-D image's two 3-tap gradient chains (cimx_edges.cu)
 int try_grad2d(const CimxArray* in, const CimxArray* out, const CimxPass* passes, int naxes,
@@ -74,7 +75,7 @@ int try_grad2d(const CimxArray* in, const CimxArray* out, const CimxPass* passes
 
 // the last two axes of a float64 array in one launch (cimx_strip_f64.cu)
 int try_strip_f64(const PassDesc& dy, const PassDesc& dx, const void* in, void* out,
-                  cudaStream_t st);
+                  cudaStream_t st, bool no_scratch);
 
 // elementwise copy with conversion (used when a filter has no passes)
 int launch_copy_cast(const void* in, int tin, void* out, int tout, int64_t n,

@@ -12,6 +12,8 @@
 // beyond (a row loads its halo again once per 240 columns). 2003 x 3001, 17 taps:
 // 34.8 us a call against 86.1 in two launches of the generic kernels, whose taps
 // and inputs all come from shared memory.
+#include <cmath>
+
 #include "cimx_strip.cuh"
 
 namespace cimx {
@@ -207,16 +209,40 @@ int launch(const PassDesc& dy, const PassDesc& dx, const void* in, void* out, cu
 
 }  // namespace strip64
 
+namespace strip64 {
+
+// Whether the strip beats the two launches of the generic kernels. Up to 25 taps
+// always, beyond, one CTA per SM, by the two costs in us of 2^24 elements at 33
+// taps (longer filters scale both alike): the strip's staged columns and rows (a
+// slab's window, its last group) against the generic tiles' rows and columns.
+// Measured, strip against generic: slabs of 8 x 256 (two CTAs side by side) 745 /
+// 884, 20 x 256 505 / 443, 64 x 256 288 / 241, 512 x 256 265 / 243, 64 x 280 296 /
+// 313, 64 x 450 (three) 275 / 256, 512 x 450 222 / 253, 20 x 64 976 / 728, 512 x 64
+// 441 / 525, 64 x 1000 213 / 241. Small arrays: the launch saved counts.
+inline bool pays(int KT, double B, double Y, double X) {
+  if (KT < 33 || B * Y * X < (1 << 19)) return true;
+  const double most = (kThreads - (KT - 1)) / kP * kP;
+  const double staged = kThreads * std::ceil(X / most) / X;
+  const double strip = 40 + (95 * kG * std::ceil(Y / kG) + 2240) / Y * staged;
+  const double generic = 45 + 94 * 64 * std::ceil(Y / 64) / Y + 92 * 256 * std::ceil(X / 256) / X;
+  return strip < generic;
+}
+
+}  // namespace strip64
+
 // The passes dy, dx along the last two axes of a float64 array with float64
-// taps. Declined: unequal tap bounds, zero taps that are left out, few rows.
+// taps. Declined: unequal tap bounds, zero taps that are left out, few rows, and
+// (but for no_scratch: the generic kernels take a scratch array) what pays()
+// leaves to the generic kernels.
 int try_strip_f64(const PassDesc& dy, const PassDesc& dx, const void* in, void* out,
-                  cudaStream_t st) {
+                  cudaStream_t st, bool no_scratch) {
   using namespace strip64;
   const int K = std::max(dy.K, dx.K);
   if (!dy.w64 || !dx.w64 || K > kMaxK || dy.L < kG || dx.L < 32) return CIMX_FUSED_DECLINED;
   if (dy.L >= (1LL << 30) || dx.L >= (1LL << 30)) return CIMX_FUSED_DECLINED;
   auto bound = [](int k) { return k <= 9 ? 9 : (k + 6) / 8 * 8 + 1; };
   if (bound(dy.K) != bound(dx.K)) return CIMX_FUSED_DECLINED;
+  if (!no_scratch && !pays(bound(K), dy.outer, dy.L, dx.L)) return CIMX_FUSED_DECLINED;
   for (const PassDesc* d : {&dy, &dx}) {
     if (d->anchor < 0 || d->anchor >= d->K) return CIMX_FUSED_DECLINED;
     for (int k = 0; k < d->K && d->skip_zero; ++k)

@@ -142,8 +142,8 @@ def test_base_alignment(ndi, pair, offset):
 
 
 def test_long_tail_passes_without_scratch_memory(ndi):
-    """Tail passes too long to share a launch take scratch memory; where there
-    is none they run as one launch all the same."""
+    """Tail passes that run faster apart take scratch memory; where there is none
+    they run as one launch all the same."""
     import ctypes
 
     from cucim_b200 import _lib
@@ -159,6 +159,9 @@ def test_long_tail_passes_without_scratch_memory(ndi):
             _run(ndi, _data((3, 40, 70), "float32"),
                  [(1, _taps(ky, "centre"), "reflect", 0), (2, _taps(kx, "holes"), "wrap", 0)],
                  "float32")
+        x = np.random.default_rng(1).standard_normal((700, 12, 64))
+        w = _taps(33, "plain")
+        _run(ndi, x, [(1, w, "reflect", 0), (2, w, "wrap", 0)], "float64")
     finally:
         set_allocator(None, None, None)
 
@@ -197,3 +200,14 @@ def test_float64_tail_passes(ndi, K, shape):
         _run(ndi, x, [(nd - 2, w, mode, 0), (nd - 1, w, mode, 0)], "float64", cval=1.25)
         _run(ndi, y, [(nd - 2, v, mode, (v.size - 1) // 2), (nd - 1, w, mode, -(K // 2))],
              "float64", cval=np.inf)
+
+
+@pytest.mark.parametrize("K", [25, 33, 49])
+@pytest.mark.parametrize("shape", [(700, 12, 63), (300, 12, 256), (20, 256, 127), (40, 65, 480)])
+def test_float64_tail_passes_large(ndi, K, shape):
+    """Larger float64 arrays on both sides of the rule between the strip and the
+    generic kernels."""
+    x = np.random.default_rng(K).standard_normal(shape)
+    w = _taps(K, "plain")
+    for mode in ("mirror", "constant"):
+        _run(ndi, x, [(1, w, mode, 0), (2, w, mode, 0)], "float64", cval=-0.5)
