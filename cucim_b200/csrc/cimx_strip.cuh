@@ -628,6 +628,13 @@ static_assert(smem_bytes<kLongMaxK>(kLongThreads) <= 48 * 1024 &&
                   smem_bytes<kSlabMaxK>(kStripThreads) <= 48 * 1024,
               "no opt-in shared memory");
 
+// choose_chunk for a grid whose y extent, 65535 at most, counts the chunks
+inline int choose_chunk_y(long long rows, double cols, double slots, int G, double per_row,
+                          double lead) {
+  const long long least = ((rows + 65534) / 65535 + G - 1) / G * G;
+  return std::max(choose_chunk(rows, cols, slots, G, per_row, lead), static_cast<int>(least));
+}
+
 template <class T, class D, int KY, int KX, int NP, bool GEN, bool SHORT = false>
 int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
   static_assert(!SHORT || KY == kShortTaps, "table size");
@@ -764,11 +771,10 @@ int launch_columns_k(const PassDesc& d, const float* w, int K, int anchor, bool 
   };
   thread_local Shape last{};
   if (last.gx != gx || last.L != d.L || last.K != K)
-    last = Shape{gx, d.L, K, choose_chunk(d.L, (double)gx, 148.0 * occ, G, K + 4, 3.0 * K + 80)};
+    last = Shape{gx, d.L, K, choose_chunk_y(d.L, (double)gx, 148.0 * occ, G, K + 4, 3.0 * K + 80)};
   a.chunk = last.chunk;
-  const long long gy = (d.L + a.chunk - 1) / a.chunk;
-  if (gx > 0x7fffffffLL || gy > 65535) return CIMX_FUSED_DECLINED;
-  const dim3 grid((unsigned)gx, (unsigned)gy);
+  if (gx > 0x7fffffffLL) return CIMX_FUSED_DECLINED;
+  const dim3 grid((unsigned)gx, (unsigned)((d.L + a.chunk - 1) / a.chunk));
   kern<<<grid, kColThreads, 0, st>>>(a);
   return cuda_fail(cudaGetLastError(), "column pass launch");
 }

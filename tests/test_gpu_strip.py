@@ -211,3 +211,18 @@ def test_float64_tail_passes_large(ndi, K, shape):
     w = _taps(K, "plain")
     for mode in ("mirror", "constant"):
         _run(ndi, x, [(1, w, mode, 0), (2, w, mode, 0)], "float64", cval=-0.5)
+
+
+def test_column_pass_along_sixty_million_samples(ndi):
+    """More rows than a grid's y extent has short chunks for: compared with the
+    oracle at both ends and in the middle."""
+    K, n = 45, 62_000_000
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x = torch.randint(0, 256, (n, 32), device="cuda", generator=g, dtype=torch.uint8)
+    w = _taps(K, "plain")
+    got = ndi.correlate1d(x, w, 0, mode="reflect")
+    for lo in (0, n // 2, n - 3000):
+        part = R.correlate1d(x[lo:lo + 3000].cpu().numpy(), w, 0, mode="reflect")
+        a = 0 if lo == 0 else K
+        b = 3000 if lo == n - 3000 else 3000 - K
+        np.testing.assert_array_equal(got[lo + a:lo + b].cpu().numpy(), part[a:b])
