@@ -170,7 +170,8 @@ int launch_ring_k(const PassDesc& d, const float* w, int K, int anchor, bool ski
   a.tiles = static_cast<int>((d.inner + kCols - 1) / kCols);
   const long long gx = a.tiles * d.outer;
   // a row costs K and its load and store, the start of a chunk its rows' loads
-  a.chunk = strip::choose_chunk_y(d.L, (double)gx, 148.0 * 3, kRows, K + 8, 4.0 * K + 1000);
+  a.chunk = strip::choose_chunk_y(d.L, (double)gx, 148.0 * 3, kRows, K + 8, 4.0 * K + 1000,
+                                  1 << 30);
   if (gx > 0x7fffffffLL) return CIMX_FUSED_DECLINED;
   kern<<<dim3((unsigned)gx, (unsigned)((d.L + a.chunk - 1) / a.chunk)), kThreads, smem, st>>>(a);
   return cuda_fail(cudaGetLastError(), "ring pass launch");

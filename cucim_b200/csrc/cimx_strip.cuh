@@ -42,6 +42,7 @@
 #include <algorithm>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "cimx_common.cuh"
 #include "cimx_fast.cuh"
@@ -475,24 +476,31 @@ __global__ void __launch_bounds__(SHORT ? kShortThreads : kStripThreads,
 constexpr int kColThreads = 128;
 constexpr int col_ctas(int KT) { return KT <= 17 ? 8 : KT <= 33 ? 6 : KT <= 49 ? 5 : 4; }
 
-template <int KT>
+template <int KT, int V>
 struct ColArgs {
   const void* in;
   void* out;
-  long long inner, columns;  // columns: outer * inner
+  long long inner, columns;  // columns: outer * inner / V
   int L, chunk, anchor, mode;
   double cval;
   int cin, dt;
   int trunc;
-  SlotTaps<KT, float> y;  // in the last slots
+  SlotTaps<KT, std::conditional_t<V == 2, f2, float>> y;  // in the last slots
 };
 
-template <class T, class D, int KT, int NP, bool GEN, int G>
+// V: adjacent columns per thread, 2 for up to 5 taps of 8- and 16-bit values to
+// float32 on aligned pairs, where loads of a byte or two per lane hold the SM's
+// load path (256 x 1024^2 uint8 / uint16, 3 taps along axis 0: 250 / 273 us, with
+// one column 316 / 333).
+template <class T, class D, int KT, int NP, bool GEN, int G, int V>
 __global__ void __launch_bounds__(kColThreads, col_ctas(KT))
-    k_columns(const __grid_constant__ ColArgs<KT> a) {
+    k_columns(const __grid_constant__ ColArgs<KT, V> a) {
+  static_assert(V == 1 || sizeof(D) == 4, "pairs are stored as floats");
+  using Row = std::conditional_t<V == 2, typename Raw<T>::type, T>;
+  using W = std::conditional_t<V == 2, f2, float>;
   const long long column = static_cast<long long>(blockIdx.x) * kColThreads + threadIdx.x;
   if (column >= a.columns) return;  // no barrier in this kernel
-  const long long o = column / a.inner, i = column - o * a.inner;
+  const long long o = column / (a.inner / V), i = (column - o * (a.inner / V)) * V;
   const int l0 = blockIdx.y * a.chunk;
   const int n = min(a.chunk, a.L - l0);
   const float cv = fill_value<float>(a.cval, a.cin, a.dt);
@@ -500,27 +508,40 @@ __global__ void __launch_bounds__(kColThreads, col_ctas(KT))
   const T* in = static_cast<const T*>(a.in) + o * a.L * a.inner + i;
   D* out = static_cast<D*>(a.out) + (o * a.L + l0) * a.inner + i;
   // kN rows r .. into v, mapped where they lie outside the axis
+  auto row = [](const T* p) {
+    if constexpr (V == 2) return load_pair<T, true>(p, 1);
+    else return __ldg(p);
+  };
   auto load = [&](auto& v, int r) {
-    constexpr int kN = sizeof(v) / sizeof(T);
+    constexpr int kN = sizeof(v) / sizeof(Row);
     if (r >= 0 && r + kN <= a.L) {
       const T* q = in + r * a.inner;
 #pragma unroll
-      for (int g = 0; g < kN; ++g) v[g] = __ldg(q + g * a.inner);
+      for (int g = 0; g < kN; ++g) v[g] = row(q + g * a.inner);
     } else {
 #pragma unroll
-      for (int g = 0; g < kN; ++g) v[g] = __ldg(in + max(fold(r + g, a.L, a.mode), 0) * a.inner);
+      for (int g = 0; g < kN; ++g) v[g] = row(in + max(fold(r + g, a.L, a.mode), 0) * a.inner);
     }
   };
   // the value of a loaded row: the fill value outside in constant mode
-  auto value = [&](T v, int r) {
-    const float x = fast::exact_float(v);
-    return fills && static_cast<unsigned>(r) >= static_cast<unsigned>(a.L) ? cv : x;
+  auto value = [&](Row v, int r) {
+    const bool outside = fills && static_cast<unsigned>(r) >= static_cast<unsigned>(a.L);
+    if constexpr (V == 2) {
+      return outside ? pack2(cv, cv) : widen<T>(v);
+    } else {
+      const float x = fast::exact_float(v);
+      return outside ? cv : x;
+    }
   };
-  float win[KT + G - 1];
-  T next[G];
+  auto store = [&](D* p, W v) {
+    if constexpr (V == 2) *reinterpret_cast<f2*>(p) = v;
+    else *p = narrow<D>(v, a.trunc);
+  };
+  W win[KT + G - 1];
+  Row next[G];
   int r = l0 - a.anchor - (KT - a.y.K);
   {
-    T first[KT - 1];
+    Row first[KT - 1];
     load(first, r);
 #pragma unroll
     for (int j = 0; j < KT - 1; ++j) win[j] = value(first[j], r + j);
@@ -532,24 +553,27 @@ __global__ void __launch_bounds__(kColThreads, col_ctas(KT))
     for (int g = 0; g < G; ++g) win[KT - 1 + g] = value(next[g], r + g);
     r += G;
     if (g0 + G < n) load(next, r);
-    float acc[G];
+    W acc[G];
 #pragma unroll
-    for (int g = 0; g < G; ++g) acc[g] = 0.f;
+    for (int g = 0; g < G; ++g) acc[g] = 0;
 #pragma unroll
     for (int k = 0; k < KT; ++k)
       if (tap_on<KT, NP, GEN, true>(k, a.y.K, a.y.centre, a.y.act)) {
 #pragma unroll
-        for (int g = 0; g < G; ++g) acc[g] = fmaf(win[g + k], a.y.w[k], acc[g]);
+        for (int g = 0; g < G; ++g) {
+          if constexpr (V == 2) acc[g] = fma2(win[g + k], a.y.w[k], acc[g]);
+          else acc[g] = fmaf(win[g + k], a.y.w[k], acc[g]);
+        }
       }
 #pragma unroll
     for (int j = 0; j < KT - 1; ++j) win[j] = win[j + G];
     if (g0 + G <= n) {
 #pragma unroll
-      for (int g = 0; g < G; ++g) out[g * a.inner] = narrow<D>(acc[g], a.trunc);
+      for (int g = 0; g < G; ++g) store(out + g * a.inner, acc[g]);
     } else {
 #pragma unroll
       for (int g = 0; g < G; ++g)
-        if (g0 + g < n) out[g * a.inner] = narrow<D>(acc[g], a.trunc);
+        if (g0 + g < n) store(out + g * a.inner, acc[g]);
     }
     out += G * a.inner;
   }
@@ -628,11 +652,13 @@ static_assert(smem_bytes<kLongMaxK>(kLongThreads) <= 48 * 1024 &&
                   smem_bytes<kSlabMaxK>(kStripThreads) <= 48 * 1024,
               "no opt-in shared memory");
 
-// choose_chunk for a grid whose y extent, 65535 at most, counts the chunks
+// choose_chunk, `most` rows at most, for a grid whose y extent, up to 65535, counts
+// the chunks
 inline int choose_chunk_y(long long rows, double cols, double slots, int G, double per_row,
-                          double lead) {
+                          double lead, int most) {
   const long long least = ((rows + 65534) / 65535 + G - 1) / G * G;
-  return std::max(choose_chunk(rows, cols, slots, G, per_row, lead), static_cast<int>(least));
+  return std::max(std::min(choose_chunk(rows, cols, slots, G, per_row, lead), most),
+                  static_cast<int>(least));
 }
 
 template <class T, class D, int KY, int KX, int NP, bool GEN, bool SHORT = false>
@@ -738,15 +764,22 @@ int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
   return cuda_fail(cudaGetLastError(), "strip launch");
 }
 
-template <class T, class D, int KT, int NP, bool GEN>
+// Rows per chunk of up to 9 taps where there are many waves of them: HBM bound, and
+// the CTAs at work should read and write close together (100000 x 50 x 50, 3 taps,
+// chunks of 64 / 96 / 256 / 1560 rows: float32 339 / 349 / 360 / 396 us, uint8 230 /
+// 223 / 221 / 264; 256 x 1024^2 float32 360 / 356 / 364, uint16 277 / 272 / 269). Few
+// waves: whole ones (4 x 1000 x 4096, 9 taps, 31 us against 36).
+template <class D> constexpr int close_chunk() { return sizeof(D) == 4 ? 96 : 256; }
+
+template <class T, class D, int KT, int NP, bool GEN, int V = 1>
 int launch_columns_k(const PassDesc& d, const float* w, int K, int anchor, bool skip,
                      const void* in, void* out, cudaStream_t st) {
   constexpr int G = kG;
-  ColArgs<KT> a{};
+  ColArgs<KT, V> a{};
   a.in = in;
   a.out = out;
   a.inner = d.inner;
-  a.columns = d.outer * d.inner;
+  a.columns = d.outer * d.inner / V;
   a.L = static_cast<int>(d.L);
   a.anchor = anchor;
   a.mode = d.mode;
@@ -756,7 +789,7 @@ int launch_columns_k(const PassDesc& d, const float* w, int K, int anchor, bool 
   double bound = type_bound<T>();
   a.trunc = trunc_bounded<T, D>(w, K, d.mode, d.cval, bound);
   put_taps(a.y, w, K, skip, true);
-  auto* kern = k_columns<T, D, KT, NP, GEN, G>;
+  auto* kern = k_columns<T, D, KT, NP, GEN, G, V>;
   static int occ = 0;
   static std::once_flag once;
   std::call_once(once, [&] {
@@ -770,8 +803,13 @@ int launch_columns_k(const PassDesc& d, const float* w, int K, int anchor, bool 
     int K, chunk;
   };
   thread_local Shape last{};
-  if (last.gx != gx || last.L != d.L || last.K != K)
-    last = Shape{gx, d.L, K, choose_chunk_y(d.L, (double)gx, 148.0 * occ, G, K + 4, 3.0 * K + 80)};
+  if (last.gx != gx || last.L != d.L || last.K != K) {
+    constexpr int kClose = close_chunk<D>();
+    const bool close = K <= 9 && gx * ((d.L + kClose - 1) / kClose) >= 8LL * 148 * occ;
+    last = Shape{gx, d.L, K,
+                 choose_chunk_y(d.L, (double)gx, 148.0 * occ, G, K + 4, 3.0 * K + 80,
+                                close ? kClose : 1 << 30)};
+  }
   a.chunk = last.chunk;
   if (gx > 0x7fffffffLL) return CIMX_FUSED_DECLINED;
   const dim3 grid((unsigned)gx, (unsigned)((d.L + a.chunk - 1) / a.chunk));
@@ -848,7 +886,11 @@ int launch_columns_td(const PassDesc& d, const float* w, int K, int anchor, bool
     return launch_columns_k<T, D, 65, 65, true>(d, w, K, anchor, skip, in, out, st);
   }
   switch (kt_bound(sizeof(T), K)) {
-    case 5: return launch_columns_k<T, D, 5, 5, false>(d, w, K, anchor, skip, in, out, st);
+    case 5:
+      if constexpr (sizeof(T) < 4 && sizeof(D) == 4)
+        if (d.inner % 2 == 0 && aligned(in, 2 * sizeof(T)) && aligned(out, 2 * sizeof(D)))
+          return launch_columns_k<T, D, 5, 5, false, 2>(d, w, K, anchor, skip, in, out, st);
+      return launch_columns_k<T, D, 5, 5, false>(d, w, K, anchor, skip, in, out, st);
     case 9: return launch_columns_k<T, D, 9, 4, false>(d, w, K, anchor, skip, in, out, st);
 #define CIMX_KT(K_) \
   case K_: return launch_columns_k<T, D, K_, 8, false>(d, w, K, anchor, skip, in, out, st);

@@ -226,3 +226,24 @@ def test_column_pass_along_sixty_million_samples(ndi):
         a = 0 if lo == 0 else K
         b = 3000 if lo == n - 3000 else 3000 - K
         np.testing.assert_array_equal(got[lo + a:lo + b].cpu().numpy(), part[a:b])
+
+
+@pytest.mark.parametrize("dtype", ["uint8", "uint16"])
+@pytest.mark.parametrize("shape", [(1, 41, 34), (3, 7, 66), (2, 200, 258), (300, 9, 32)])
+def test_column_pairs(ndi, dtype, shape):
+    """Up to 5 taps of 8- and 16-bit values to float32 along strided axes, two
+    columns per thread on aligned pairs and one elsewhere."""
+    n = int(np.prod(shape))
+    for off_in, off_out in ((0, 0), (1, 0), (0, 1), (2, 2)):
+        flat = _data(n + 2, dtype, n + off_in)
+        x, xd = flat[off_in:off_in + n].reshape(shape), torch.as_tensor(flat).cuda()
+        xd = xd[off_in:off_in + n].view(shape)
+        out = torch.empty(n + 2, device="cuda")[off_out:off_out + n].view(shape)
+        for K, kind in ((1, "plain"), (2, "signed"), (3, "centre"), (4, "plain"), (5, "signed")):
+            w = _taps(K, kind)
+            for mode in MODES:
+                for ax in (0, 1):
+                    ndi.correlate1d(xd, w, ax, out, mode, 3.0, origin=-((K - 1) // 2))
+                    exp = R.correlate1d(x, w, ax, output=np.dtype(np.float32), mode=mode,
+                                        origin=-((K - 1) // 2), cval=3.0)
+                    np.testing.assert_array_equal(out.cpu().numpy(), exp)
