@@ -213,15 +213,14 @@ def step_ops(ndi, x, outs):
         op(ndi, x, o)
 
 
-# gaussian: one streamed z pass + one fused (y, x) launch; each sobel and the
+# gaussian: one column launch (z) + one strip launch (y, x); each sobel and the
 # uniform filter: one launch of the volume kernel
 LAUNCHES_PER_STEP = 6
 
 # DRAM bytes per launch measured by ncu on a smaller stack: (bytes, slices of
 # that stack, profile file)
 TRAFFIC = {
-    "slab f32->f32 gaussian y,x K=17,17": (201.404672e6 + 162.276608e6, 48,
-                                           "k_slab_f32_gaussian_yx_48x1024x1024_and_2048x2048.md"),
+    "strip f32->f32 gaussian y,x K=17,17": (494.891e6, 64, "strip_column_ring_tile_kernels.md"),
     "volume u16->f32 sobel K=3,3,3": (135.097344e6 + 212.728064e6, 64,
                                       "k_vol_u16_f32_sobel_64x1024x1024.md"),
 }
@@ -307,12 +306,12 @@ def run_ours(args, rank, world, local_rank):
     kt = {
         "volume u16->f32 sobel K=3,3,3": (
             lambda: ndi.sobel(x, 0, output=outs[1]), 6 * nvox, 3),
-        "slab f32->f32 gaussian y,x K=17,17": (
+        "strip f32->f32 gaussian y,x K=17,17": (
             lambda: ndi.gaussian_filter(tmp, (0, 2, 2), mode="mirror", output=outs[1]),
             8 * nvox, 1),
         "volume u16->u16 uniform K=5,5,5": (
             lambda: ndi.uniform_filter(x, 5, output=outs[4]), 4 * nvox, 1),
-        "stream u16->f32 gaussian z K=9": (
+        "columns u16->f32 gaussian z K=9": (
             lambda: ndi.gaussian_filter1d(x, 1.0, axis=0, mode="mirror", output=outs[1]),
             6 * nvox, 1),
     }

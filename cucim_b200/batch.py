@@ -4,7 +4,7 @@ this library; cuCIM runs `color.rgb2gray`, `filters.gaussian` and
 `filters.sobel` once per tile).
 
     batch = TileBatch(rgb_tiles, sigmas)     # prepares the device tables once
-    batch.run()                              # one persistent launch
+    batch.run()                              # one launch
     g = batch.graph(); g.replay()            # the same launch in a CUDA graph
     batch.outputs                            # float32 tiles, bit-identical to
                                              # sobel(gaussian(rgb2gray(t), s))

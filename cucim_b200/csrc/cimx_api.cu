@@ -276,10 +276,13 @@ int cimx_separable(const CimxArray* in, const CimxArray* out, const CimxPass* pa
 
   const bool tf32x3 = (lib_flags & CIMX_L_TENSOR_TF32X3) != 0;
   const bool tensor = tf32x3 || (lib_flags & CIMX_L_TENSOR_BF16X3) != 0;
-  // Tensor-core passes where they measured faster than the plain kernels: on
-  // a B200, 1.2-2.3x for 23-143 taps along 8192-sample lines, slower or even
-  // for every length along 256-sample lines (the band's halo and the strip
-  // set-up dominate short lines). CIMX_L_TENSOR_ALL_LINES lifts the limit.
+  // Where the caller's opt-in takes the tensor cores. Short lines never pay (the
+  // band's halo and the strip set-up dominate along 256 samples). The tap limit
+  // is older than the strip and ring kernels, which are the faster ones up to
+  // 105-129 taps: 8192^2, axis 0 / 1, TF32x3 against plain float32, us: 41 taps
+  // 193 / 204 against 133 / 143, 81 261 / 274 against 220 / 230, 129 304 / 312
+  // against 320 / 301, 143 486 / 493 against 583 / 748, 257 606 / 601 against 899 /
+  // 1171; the autotuner tries both. CIMX_L_TENSOR_ALL_LINES lifts the line limit.
   constexpr int64_t kTensorMinLine = 2048;
   const bool all_lines = (lib_flags & CIMX_L_TENSOR_ALL_LINES) != 0;
   auto tensor_kind = [&](const PassDesc& d) {
@@ -334,8 +337,7 @@ int cimx_separable(const CimxArray* in, const CimxArray* out, const CimxPass* pa
       // a pass list the fused kernels do not take as a whole (axes out of
       // ascending order, as the edge filters' edge-then-smooth chains along
       // axis 1 or 2): each pass on its own still runs on a fast kernel when
-      // one covers it (the stream kernel for a leading axis, the slab for a
-      // pass along the second-to-last axis), the same chain as the generic
+      // one covers it (column, ring or strip), the same chain as the generic
       // kernel. CIMX_L_NO_FUSION keeps the generic kernels.
       rc = CIMX_FUSED_DECLINED;
       if (!(lib_flags & CIMX_L_NO_FUSION)) {

@@ -4,7 +4,9 @@
 //
 // Each kernel evaluates the same expression, statement by statement, as the
 // cuCIM kernel it replaces (cited per kernel), so the compiler's rounding and
-// contraction decisions are the same ones cuCIM's kernels get.
+// contraction decisions are the same ones cuCIM's kernels get. Two exceptions, for
+// float32 results alone, whose rounding hides the difference: eig33's cosines and
+// the vesselness' quotients (frangi_quotient).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>

@@ -4,7 +4,7 @@
 #pragma once
 
 #include "cimx_common.cuh"
-#include "cimx_tma.cuh"
+#include "cimx_tma.cuh"  // smem_addr
 
 namespace cimx {
 namespace fast {

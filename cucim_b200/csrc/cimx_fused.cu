@@ -124,7 +124,13 @@ int launch_vol(const VolArgs& v, int tin, int tout, cudaStream_t st) {
 }
 
 // z, y and x passes over the last three axes with the same short taps: one
-// launch of the volume kernel, no intermediate volume
+// launch of the volume kernel, no intermediate volume. Against a column and a strip
+// launch (CIMX_L_NO_VOLUME), us: 256 x 1024^2, 3 taps float32 506 / 733, uint16 to
+// float32 484 / 647, uint16 540 / 660, uint8 530 / 612; 203 x 1021 x 1016 uint16 418
+// / 541. With 5 taps it keeps the float32 volumes (671 / 733) but for 512^3 (411 /
+// 381) and loses the integer ones (uint16 707 / 654, uint8 717 / 637, uint16 to
+// float32 684 / 644), like 3 taps with a zero centre to integers (uint16 768 / 675):
+// left to the autotuner, which tries both.
 int try_vol(const CimxArray* in, const CimxArray* out, const PassDesc* ds, int zchunk,
             cudaStream_t st) {
   const int nd = in->ndim;

@@ -14,7 +14,8 @@ namespace cimx {
 constexpr int CIMX_FUSED_DECLINED = 1;
 
 constexpr int kSlabMaxK = 65;   // longest pass the strip and column kernels take
-constexpr int kLongMaxK = 129;  // the same for a float32 pass of its own
+constexpr int kLongMaxK = 129;  // the same for a float32 pass of its own: as far as
+                                // k_ring and k_strip are instantiated
 
 // One pass of the strip and volume kernels (float32 weights, already trimmed).
 struct SlabPass {

@@ -33,10 +33,10 @@
 // alone, 256^3 float32, 17 / 57 taps: 33 / 53 against 65 / 156; 8192^2, 129 taps
 // 293 us (82 % of the FMA rate) against 699 on k_rows (taps in shared memory).
 //
-// Also measured: one column per thread with scalar FMAs, which doubles the
-// warps: 364 instead of 294 us at 128 x 1024^2, 17 taps (twice the shared
-// reads per FMA); taps in shared memory 324 instead of 279; a transposed FIR
-// (chains in registers instead of inputs) spilled at every tap count.
+// Also measured, against the kernel as it then was at 128 x 1024^2, 17 taps: one
+// column per thread with scalar FMAs, which doubles the warps, 1.24 times as long
+// (twice the shared reads per FMA); taps in shared memory 1.16 times; a transposed
+// FIR (chains in registers instead of inputs) spilled at every tap count.
 #pragma once
 
 #include <algorithm>
@@ -96,7 +96,9 @@ __device__ __forceinline__ f2 widen(typename Raw<T>::type r) {
 
 // map_coord by repeated folding: the same index without a division, whose
 // inlined code costs these kernels registers. An overhang takes one turn per
-// axis length, and it is shorter than the taps.
+// axis length: of a row, fewer than the taps; of a column, up to the staged
+// columns of the CTA (rows of 2, 64 turns: slabs of 64 x 2, 9 taps, 1.9 ms for
+// 2^24 float32, on the generic kernels 14).
 __device__ __forceinline__ int fold(int i, int n, int mode) {
   if (static_cast<unsigned>(i) < static_cast<unsigned>(n)) return i;
   if (mode == CIMX_MODE_CONSTANT) return -1;

@@ -26,7 +26,7 @@ using strip::tap_on;
 constexpr int kThreads = 256;
 constexpr int kG = 8;   // rows per group
 constexpr int kP = 8;   // x outputs per thread
-constexpr int kMaxK = 49;
+constexpr int kMaxK = 49;  // instantiated up to here: 182 registers, two more per tap
 constexpr int ctas(int KT) { return KT <= 25 ? 2 : 1; }
 
 // bytes per staged row, 16 modulo 128: the rows of 8 lanes hit distinct banks

@@ -88,8 +88,8 @@ def _build_passes(in_dtype, out_dtype, ndim, specs, cval, algorithm):
 
 # algorithm="tensor" and "tensor_bf16x3": additions of this library (cuCIM
 # accepts only "shared_memory", "elementwise" and None). float32 -> float32
-# passes with at least 16 taps along lines of at least 2048 samples (where
-# they measured faster; see tensor_cores_everywhere) run on the tensor cores
+# passes with at least 16 taps along lines of at least 2048 samples (see
+# tensor_cores_everywhere) run on the tensor cores
 # as banded-Toeplitz products with float32 accumulation: "tensor" splits operands into tf32
 # hi + lo (TF32x3, max relative error near 1e-6), "tensor_bf16x3" into
 # bfloat16 hi + lo (BF16x3, near 1e-5). Results are close to, not
@@ -121,7 +121,7 @@ def pass_by_pass():
 @contextlib.contextmanager
 def schedule(lib_flags):
     """Within this block every filter runs with the given CIMX_L_* schedule
-    flags (for example _lib.L_NO_VOLUME | _lib.L_NO_ROWSTREAM), which the
+    flags (for example _lib.L_NO_VOLUME | _lib.L_NO_STREAM), which the
     autotuner then leaves alone. All schedules give bit-identical results;
     a testing and measurement aid, not thread-safe."""
     global _EXTRA_LIB_FLAGS
@@ -162,7 +162,7 @@ def tensor_cores_everywhere():
     """Within this block algorithm="tensor" / "tensor_bf16x3" runs every
     eligible pass on the tensor cores, whatever its line length. By default
     only passes along lines of at least 2048 samples do (on shorter lines the
-    plain kernels measured faster). A testing and measurement aid, not
+    plain kernels are faster at any length; on longer ones, up to 105-129 taps). A testing and measurement aid, not
     thread-safe."""
     global _EXTRA_LIB_FLAGS
     old = _EXTRA_LIB_FLAGS

@@ -519,8 +519,8 @@ typedef struct CimxBatchTile {
  * _shared/filters.py:21-166), then the sobel gradient magnitude with mode
  * 'reflect' (filters/edges.py:148-306: edge taps `edge_taps` along one axis,
  * `smooth_taps` along the other, both as correlation taps after the
- * convolution flip), float32 out — one persistent launch over the tiles'
- * 64 x 64 output blocks (`nblocks` in all). Results are bit-identical to the
+ * convolution flip), float32 out — one launch over strips of the tiles, whose
+ * table counts 64 x 64 output blocks (`nblocks` in all). Results are bit-identical to the
  * three per-tile calls. `tiles` and `taps` are device memory prepared by the
  * caller, so the launch can be captured in a CUDA graph and replayed;
  * `edge_taps` and `smooth_taps` are 3 host floats read at the call.

@@ -1,9 +1,9 @@
 """The generic row and column kernels and lone passes along the last axis
 (correlate1d / convolve1d /
 gaussian_filter1d / uniform_filter1d along axis -1, and filters whose only
-pass besides the last axis is a leading one). Over float32 data the slab
-kernel takes such a pass behind an identity y pass; every other pair runs
-on the generic row kernel (typed or runtime-typed loads, outputs stored
+pass besides the last axis is a leading one). The strip kernel takes such a
+pass over float32 and 8/16-bit data behind an identity y pass; every other pair
+runs on the generic row kernel (typed or runtime-typed loads, outputs stored
 straight or through the row buffer by their width). Either way the result
 must equal the oracle bit for bit (cuCIM's
 _vendored/_ndimage_filters.py:109-134 per pass) and the one-launch-per-pass
@@ -104,7 +104,7 @@ def test_uniform_last_axis(ndi, tin, tout, size):
 @pytest.mark.parametrize("tin,tout", PAIRS[:5])
 @pytest.mark.parametrize("sigma", [(1.0, 0, 2.0), (0, 0, 1.5), (2.0, 0.0, 0.7)])
 def test_leading_pass_then_last_axis(ndi, tin, tout, sigma):
-    """A z pass (stream kernel) followed by the last axis alone."""
+    """A z pass (column kernel) followed by the last axis alone."""
     x = _input((12, 20, 72), tin, 4)
     xd = dev(x)
     got = host(ndi.gaussian_filter(xd, sigma, mode="reflect", output=tout))
@@ -127,7 +127,7 @@ def test_last_axis_non_finite_and_signed_zero(ndi):
 
 
 def test_last_axis_large_rows(ndi):
-    """Rows longer than one slab tile and many slabs per CTA."""
+    """Rows over many strips."""
     x = _input((40, 24, 3000), np.uint16, 6)
     xd = dev(x)
     got = host(ndi.gaussian_filter1d(xd, 2.0, axis=-1, output=np.float32))
@@ -164,11 +164,9 @@ def test_strided_axes_generic(ndi, tin, tout, mode):
                                          ("constant", "constant"), ("wrap", "nearest"),
                                          ("mirror", "reflect"), ("nearest", "wrap")])
 def test_integer_slab_modes(ndi, tin, tout, ymode, xmode):
-    """The (y, x) slab kernel on 8/16-bit input with TMA-eligible rows (a
-    multiple of 16 bytes): tiles inside the array and tiles past every edge,
-    one mode per axis, a fill value that does not fit the input dtype; the
-    y pass reads the raw tile directly except where rows outside take a
-    constant fill."""
+    """The (y, x) strip kernel on 8/16-bit input: strips inside the array and
+    past every edge, one mode per axis, a fill value that does not fit the input
+    dtype."""
     x = _input((2, 70, 272), tin, 8)
     xd = dev(x)
     for sigma in ((0, 0.7, 1.2), (0, 2.0, 4.0), (0, 5.0, 1.0)):

@@ -1,8 +1,7 @@
 """The autotuner on the GPU: tuning a call signature records one table
 entry, and the result of the tuned schedule is bit-identical to the oracle
-and to every forced schedule (volume kernel or not, stream or generic
-leading passes, row stream or slab, z chunks, slabs per CTA, one launch
-per pass). A later
+and to every forced schedule (volume kernel or not, column or generic
+leading passes, z chunks, one launch per pass). A later
 call of the same signature uses the entry without timing again. With
 algorithm="tensor" the tuner may also pick the plain passes; either result
 stays within the tensor path's tolerance."""
@@ -26,9 +25,9 @@ def mods(cuda):
 
 def _schedules(lib):
     z, sp = lib.L_ZCHUNK_SHIFT, lib.L_SLAB_SPAN_SHIFT
-    return [lib.L_NO_FUSION, lib.L_NO_VOLUME, lib.L_NO_ROWSTREAM, lib.L_NO_STREAM,
-            lib.L_NO_VOLUME | lib.L_NO_ROWSTREAM, lib.L_NO_VOLUME | lib.L_NO_STREAM,
-            1 << z, 2 << z, 3 << z, 1 << sp, 2 << sp, 3 << sp,
+    return [lib.L_NO_FUSION, lib.L_NO_VOLUME, lib.L_NO_STREAM,
+            lib.L_NO_VOLUME | lib.L_NO_STREAM, 1 << z, 2 << z, 3 << z,
+            # flags of earlier recordings, which have no effect
             lib.L_NO_VOLUME | lib.L_NO_ROWSTREAM | (3 << sp)]
 
 
@@ -51,6 +50,13 @@ WORKLOADS = [
      lambda f, x: f.gaussian_filter(x, 4.0, mode="reflect")),
     ("gaussian f32 3-D sigma 3", lambda: _f32((20, 40, 64), 5),
      lambda f, x: f.gaussian_filter(x, 3.0)),
+    # both tail passes in a strip launch, apart, and the z pass on the ring kernel
+    ("gaussian f32 3-D, tails apart", lambda: _f32((60, 70, 64), 7),
+     lambda f, x: f.gaussian_filter(x, (4.0, 5.0, 1.0))),
+    ("gaussian u16->f32 3-D, tails apart", lambda: _u16((20, 60, 50), 8),
+     lambda f, x: f.gaussian_filter(x, (1.0, 6.0, 3.0), output=np.float32)),
+    ("gaussian f64 2-D", lambda: _f32((90, 70), 9).astype(np.float64),
+     lambda f, x: f.gaussian_filter(x, 2.0)),
     ("prewitt u8->u8 3-D", lambda: _u16((12, 33, 40), 6).astype(np.uint8),
      lambda f, x: f.prewitt(x, 0)),
 ]

@@ -1,7 +1,7 @@
 """The fused kernels of the plain path on rows of a multiple of 4 elements
 (the vector kernels' condition): the single-launch 3-D kernel (3 or 5 taps
 on each of the last three axes: z, y and x passes in one launch) and the
-(y, x) slab kernel with 9 or 17 taps. Their outputs must be bit-identical
+(y, x) strip kernel with 9 or 17 taps. Their outputs must be bit-identical
 to the oracle and to the pass-by-pass schedule (one launch per pass through
 a scratch volume). The shapes cover partial tiles in y and x, short and
 chunked z, a leading batch axis and rows of only 8 elements."""
@@ -151,8 +151,7 @@ def test_narrowed_intermediates_2d(ndi, shape, tout):
     """Sobel of uint8 into uint8 / uint16: the first pass's negative and
     out-of-range values are narrowed as cast<D>() stores them (wrap for
     negatives, saturation above the range) before the next pass reads them,
-    also where the intermediate never leaves the chip (row-streaming and
-    slab kernels)."""
+    also where the intermediate never leaves the chip (the strip kernel)."""
     x = _ints(shape, np.uint8, 11, hi=256)
     xd = dev(x)
     for axis in range(len(shape)):
@@ -220,8 +219,8 @@ def test_slab_long_taps_match_pass_by_pass(ndi):
 
 @pytest.mark.parametrize("mode", ["mirror", "constant", "wrap"])
 def test_long_leading_pass_then_slab(ndi, mode):
-    # the z pass is longer than the stream kernel takes (25 taps): it runs on
-    # the generic kernel, the (y, x) passes still as one slab launch
+    # a long z pass (25 taps) on its own column or ring launch, the (y, x)
+    # passes as one strip launch
     x = np.random.default_rng(23).standard_normal((30, 70, 136)).astype(np.float32)
     xd = dev(x)
     got = ndi.gaussian_filter(xd, (3.0, 2.0, 1.5), mode=mode, cval=0.5)
@@ -274,9 +273,9 @@ def test_passes_out_of_axis_order(ndi, axes, tin, tout):
                                       (np.float32, np.float32), (np.uint8, np.uint8)])
 @pytest.mark.parametrize("mode", MODES)
 def test_stream_tap_counts(ndi, taps, tin, tout, mode):
-    """A pass along a leading axis at every tap count the stream kernel is
-    instantiated for (19 and above: the generic kernel), uneven
-    taps with an origin, against the oracle and the generic schedule."""
+    """A pass along a leading axis on the column kernel at odd tap counts up to
+    25, uneven taps with an origin, against the oracle and the generic
+    schedule."""
     x = _ints((23, 6, 40), tin, 30 + taps, hi=250)
     w = np.linspace(-0.4, 0.9, taps)
     origin = (taps - 1) // 2 - taps // 3
