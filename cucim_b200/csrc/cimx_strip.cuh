@@ -286,11 +286,17 @@ struct StripArgs {
   int cin_y, cin_x, dt_y, dt_x;
   int trunc;           // truncating narrowing casts (narrow())
   int add;             // float32: out += the result instead of out = it
-  int group;           // SHORT: rows per group, whole slabs
-  short src[kG * kShortTaps];  // SHORT: row of the group that [row][y tap slot] reads, -1: fill
   SlotTaps<KY, f2> y;  // in the last slots
   SlotTaps<KX, f2> x;  // in the first slots
 };
+
+template <int KY, int KX>
+struct ShortArgs : StripArgs<KY, KX> {
+  int group;                   // rows per group, whole slabs
+  short src[kG * kShortTaps];  // row of the group that [row][y tap slot] reads, -1: fill
+};
+template <int KY, int KX, bool SHORT>
+using StripKernelArgs = std::conditional_t<SHORT, ShortArgs<KY, KX>, StripArgs<KY, KX>>;
 
 //
 // SHORT: slabs of up to kG rows and up to kShortTaps taps. A group of kG rows
@@ -305,7 +311,7 @@ struct StripArgs {
 template <class T, class D, int KY, int KX, int NP, bool GEN, bool SHORT>
 __global__ void __launch_bounds__(SHORT ? kShortThreads : kStripThreads,
                                   SHORT ? 6 : strip_ctas<T>(KY))
-    k_strip(const __grid_constant__ StripArgs<KY, KX> a) {
+    k_strip(const __grid_constant__ StripKernelArgs<KY, KX, SHORT> a) {
   extern __shared__ __align__(16) unsigned char sm_strip[];
   const int t = threadIdx.x, NT = blockDim.x;
   const int tile = blockIdx.x % a.tiles_x, ch = blockIdx.x / a.tiles_x;
@@ -333,7 +339,8 @@ __global__ void __launch_bounds__(SHORT ? kShortThreads : kStripThreads,
   const unsigned char* win0 = sm_strip + (xwork ? rp : 0) * rs + cg * mid_off(kP);
   unsigned char* put0 = sm_strip + mid_off(2 * t);
   const int xo = x0 + cg * kP;
-  const int group = SHORT ? a.group : kG;
+  int group = kG;
+  if constexpr (SHORT) group = a.group;
   f2* const own = reinterpret_cast<f2*>(sm_strip + 2 * kRP * rs) + t;  // SHORT: [row * NT]
 
   for (long long b = blockIdx.y; b < a.B; b += gridDim.y) {
@@ -353,8 +360,7 @@ __global__ void __launch_bounds__(SHORT ? kShortThreads : kStripThreads,
         win[i + g] = (fill >> g) & 1u ? pack2(cy, cy) : widen<T>(next[g]);
     }
     r += KY - 1;  // row of next[0]
-    const int my = SHORT ? CIMX_MODE_NEAREST : a.my;
-    uint32_t fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, my);
+    uint32_t fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, SHORT ? CIMX_MODE_NEAREST : a.my);
 
     int par = 0;
     for (int g0 = 0; g0 < n; g0 += group, par ^= 1) {
@@ -416,7 +422,8 @@ __global__ void __launch_bounds__(SHORT ? kShortThreads : kStripThreads,
       }
 #pragma unroll
       for (int i = 0; !SHORT && i < KY - 1; ++i) win[i] = win[i + kG];
-      if (g0 + group < n) fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, my);
+      if (g0 + group < n)
+        fill = load_rows<T>(next, in, d1, vec, r, a.Y, a.X, SHORT ? CIMX_MODE_NEAREST : a.my);
       __syncthreads();
       if (xwarp) {
         const unsigned char* src = win0 + par * kRP * rs;
@@ -664,18 +671,13 @@ inline int choose_chunk_y(long long rows, double cols, double slots, int G, doub
 }
 
 template <class T, class D, int KY, int KX, int NP, bool GEN, bool SHORT = false>
-int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
+int launch_strip_k(const SlabArgs& s, cudaStream_t st) {
   static_assert(!SHORT || KY == kShortTaps, "table size");
-  SlabArgs s = slabs;
-  if (SHORT) {
-    s.Y *= s.B;
-    s.B = 1;
-  }
-  StripArgs<KY, KX> a{};
+  StripKernelArgs<KY, KX, SHORT> a{};
   a.in = s.in;
   a.out = s.out;
-  a.B = s.B;
-  a.Y = static_cast<int>(s.Y);
+  a.B = SHORT ? 1 : s.B;
+  a.Y = static_cast<int>(SHORT ? s.B * s.Y : s.Y);
   a.X = static_cast<int>(s.X);
   a.ay = s.py.anchor;
   a.ax = s.px.anchor;
@@ -698,11 +700,11 @@ int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
               : a.X % 4 == 0 && aligned(a.out, 4 * sizeof(D)) ? 1
                                                                 : 0;
 
-  a.group = kG;
-  if (SHORT) {
-    const int L = static_cast<int>(slabs.Y), lead = KY - s.py.K;
-    a.group = kG / L * L;
-    for (int g = 0; g < a.group; ++g)
+  int group = kG;
+  if constexpr (SHORT) {
+    const int L = static_cast<int>(s.Y), lead = KY - s.py.K;
+    a.group = group = kG / L * L;
+    for (int g = 0; g < group; ++g)
       for (int k = 0; k < s.py.K; ++k) {
         const int m = map_coord32(g % L - s.py.anchor + k, L, s.py.mode);
         a.src[g * KY + lead + k] = static_cast<short>(m < 0 ? -1 : g / L * L + m);
@@ -728,8 +730,8 @@ int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
     int ky, kx, group, nt, xw, tiles_x, chunk;
   };
   thread_local Shape last{};
-  if (last.B != s.B || last.Y != s.Y || last.X != s.X || last.ky != a.y.K || last.kx != a.x.K ||
-      last.group != a.group) {
+  if (last.B != a.B || last.Y != a.Y || last.X != a.X || last.ky != a.y.K || last.kx != a.x.K ||
+      last.group != group) {
     // CTA width: the staged columns of all tiles together as few as possible
     int nt = 0;
     long long tiles = 0, best = 0;
@@ -739,7 +741,7 @@ int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
       // seven that stage (8192^2, 129 taps: 414 us with five)
       if (KX > kSlabMaxK) xw = std::min(xw, 256);
       if (xw < 16) continue;
-      const long long tl = (s.X + xw - 1) / xw;
+      const long long tl = (a.X + xw - 1) / xw;
       long long cost = tl * w;
       const int res = occ[w / 32] * w;  // fewer than 8 warps cannot fill the pipe
       if (res < 256) cost = cost * 256 / res;
@@ -749,19 +751,19 @@ int launch_strip_k(const SlabArgs& slabs, cudaStream_t st) {
         best = cost;
       }
     }
-    const int xw = static_cast<int>(((s.X + tiles - 1) / tiles + 15) / 16 * 16);
-    const int tiles_x = static_cast<int>((s.X + xw - 1) / xw);
-    const int chunk = choose_chunk(s.Y, (double)tiles_x * s.B, 148.0 * occ[nt / 32], a.group,
+    const int xw = static_cast<int>(((a.X + tiles - 1) / tiles + 15) / 16 * 16);
+    const int tiles_x = static_cast<int>((a.X + xw - 1) / xw);
+    const int chunk = choose_chunk(a.Y, (double)tiles_x * a.B, 148.0 * occ[nt / 32], group,
                                    a.y.K + a.x.K + 6, 4.0 * a.y.K + 150);
-    last = Shape{s.B, s.Y, s.X, a.y.K, a.x.K, a.group, nt, xw, tiles_x, chunk};
+    last = Shape{a.B, a.Y, a.X, a.y.K, a.x.K, group, nt, xw, tiles_x, chunk};
   }
   const int nt = last.nt;
   a.xw = last.xw;
   a.tiles_x = last.tiles_x;
   a.chunk = last.chunk;
-  const long long gx = ((s.Y + a.chunk - 1) / a.chunk) * a.tiles_x;
+  const long long gx = (a.Y + a.chunk - 1LL) / a.chunk * a.tiles_x;
   if (gx > 0x7fffffffLL) return CIMX_FUSED_DECLINED;
-  const dim3 grid((unsigned)gx, (unsigned)std::min<long long>(s.B, 65535));
+  const dim3 grid((unsigned)gx, (unsigned)std::min<long long>(a.B, 65535));
   kern<<<grid, nt, smem(nt), st>>>(a);
   return cuda_fail(cudaGetLastError(), "strip launch");
 }
